@@ -256,4 +256,32 @@ struct CtaTeam {
   }
 };
 
+// Permutation of the reference's DO_SORT selection sort (tql2_tiled.hpp:
+// 149-176): for distinct, non-NaN eigenvalues it is the ascending order,
+// computed here by ranks in parallel; with ties or NaNs the serial
+// first-strict-minimum/swap procedure is replayed exactly.
+template <class T>
+__device__ void select_sort_serial(const int n, T *dwork, int *pos)
+{
+  for (int i = 0; i < n; i++) pos[i] = i;
+  for (int l = 0; l < n - 1; l++) {
+    T dl = dwork[l];
+    int il = l;
+    for (int j = l + 1; j < n; j++) {
+      const T dj = dwork[j];
+      if (dl > dj) {
+        dl = dj;
+        il = j;
+      }
+    }
+    if (il != l) {
+      const int t = pos[l];
+      pos[l] = pos[il];
+      pos[il] = t;
+      dwork[il] = dwork[l];
+      dwork[l] = dl;
+    }
+  }
+}
+
 }  // namespace eigb

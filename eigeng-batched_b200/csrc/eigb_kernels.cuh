@@ -4,11 +4,17 @@
 //   k1_warp        phase 1 for n <= 32: one warp per matrix, 4 per CTA
 //   k1_cl          phase 1 for 32 < n <= 512 on a thread-block cluster, the
 //                  matrix in the cluster's distributed shared memory
-//   k1_reg<NB>     phase 1 for 32 < n <= 128: one CTA per matrix, the matrix
+//   k1_reg<NB>     phase 1 for 32 < n <= 64: one CTA per matrix, the matrix
 //                  in registers (eigb_tridiag_reg.cuh)
-//   k1_cta<SPLIT>  phase 1 for larger n: one CTA per matrix; the leading
-//                  block that fits is staged in shared memory, the rest is
-//                  reduced in place in global memory
+//   k1_sym<...>    phase 1 for n > 64, the reduction: the upper triangle in
+//                  registers and shared memory of one CTA or of a cluster
+//                  (eigb_tridiag_sym.cuh)
+//   k1_factor, k1_formq  phase 1 for n > 64, Q from the reflectors on the
+//                  FP64 tensor cores (eigb_formq.cuh)
+//   k1_cta<SPLIT>  phase 1 where the device cannot run k1_sym's cluster: one
+//                  CTA per matrix; the leading block that fits is staged in
+//                  shared memory, the rest is reduced in place in global
+//                  memory
 //   k2_ql          phase 2: QL on (d, e), one matrix per thread
 //   k3_warp        phase 3 for n <= 32: rotations applied to Q held in
 //                  registers (one row per lane), selection-sort emulation,
@@ -28,12 +34,14 @@
 
 #include "eigb_apply.cuh"
 #include "eigb_common.cuh"
+#include "eigb_formq.cuh"
 #include "eigb_ql.cuh"
 #include "eigb_symfunc.cuh"
 #include "eigb_tmem.cuh"
 #include "eigb_tridiag.cuh"
 #include "eigb_tridiag_cl.cuh"
 #include "eigb_tridiag_reg.cuh"
+#include "eigb_tridiag_sym.cuh"
 
 namespace eigb {
 
@@ -45,6 +53,8 @@ template <class T> struct KP {
   T *d, *e;      // workspace: tridiagonal, n per matrix each
   Rec<T> *rec;   // workspace: rotation records, rcap per matrix
   Meta *meta;    // workspace: per-matrix status
+  unsigned char *vw;  // workspace: reflectors and their factors in phase 1
+  size_t vstride;     // ... bytes per matrix (they share the records' place where it is large enough)
   T *zs;         // workspace: n*n per matrix when Z does not fit in shared memory
   int k1b;       // phase 1 (CTA form): leading block kept in shared memory
   int zrows;     // phase 3 with Z in shared memory: rows per CTA ...
@@ -255,6 +265,50 @@ __global__ void __launch_bounds__(32 * SPLIT, 1024 / (32 * SPLIT)) k1_cl(const K
                                reinterpret_cast<T *>(smem_raw));
 }
 
+// Reduction of k1_sym<T, NW, RS, CN>: NW warps, RS blocks of a warp in
+// registers, CN CTAs per matrix (see eigb_tridiag_sym.cuh and sym_cfg).
+template <class T, int NW, int RS, int CN, int MB>
+__global__ void __launch_bounds__(32 * NW, MB) k1_sym(const KP<T> p)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const long k = blockIdx.x / CN;
+  unsigned char *v = p.vw + (size_t)k * p.vstride;
+  tridiag_sym<T, NW, RS, CN>(mat_ptr(p, k), p.nm, p.n, p.ap ? p.ap + (size_t)k * packed_size(p.n) : nullptr,
+                             p.d + k * p.n, p.e + k * p.n, reinterpret_cast<T *>(v + fq_off_v(p.n)), fq_ldv(p.n),
+                             reinterpret_cast<double *>(v), reinterpret_cast<T *>(smem_raw));
+}
+
+// Block factors of the formation of Q, one warp per (matrix, block).
+constexpr int K1F_NW = 4;
+template <class T>
+__global__ void __launch_bounds__(32 * K1F_NW) k1_factor(const KP<T> p)
+{
+  __shared__ double gs[K1F_NW][FQ_B * (FQ_B + 1)];
+  const int nJ = fq_blocks(p.n), wid = threadIdx.x >> 5;
+  const long id = (long)blockIdx.x * K1F_NW + wid;
+  if (id >= p.Lc * nJ) return;  // uniform per warp; no CTA barrier below
+  unsigned char *v = p.vw + (size_t)(id / nJ) * p.vstride;
+  const int J = (int)(id % nJ);
+  fq_factor<T>(p.n, J, reinterpret_cast<const T *>(v + fq_off_v(p.n)), fq_ldv(p.n),
+               reinterpret_cast<const double *>(v),
+               reinterpret_cast<double *>(v + fq_off_s(p.n)) + (size_t)J * FQ_B * FQ_B, gs[wid]);
+}
+
+// Q from the reflectors, fq_rows(NCG) columns of Q per CTA.
+__host__ __device__ constexpr int fq_rows(int ncg) { return 64 / ncg; }
+template <class T, int NTL, int NCG, int MB>
+__global__ void __launch_bounds__(256, MB) k1_formq(const KP<T> p, const int nbuf)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int per = (p.n + fq_rows(NCG) - 1) / fq_rows(NCG);
+  const long k = blockIdx.x / per;
+  const unsigned char *v = p.vw + (size_t)k * p.vstride;
+  form_q<T, NTL, NCG>(mat_ptr(p, k), p.nm, p.n, (int)(blockIdx.x % per) * fq_rows(NCG),
+                      reinterpret_cast<const T *>(v + fq_off_v(p.n)), fq_ldv(p.n),
+                      reinterpret_cast<const double *>(v + fq_off_s(p.n)), nbuf,
+                      reinterpret_cast<double *>(smem_raw));
+}
+
 // ---------------------------------------------------------------- phase 2
 template <class T>
 __global__ void __launch_bounds__(K2_MAX_WARPS * 32) k2_ql(const KP<T> p)
@@ -298,35 +352,6 @@ __global__ void __launch_bounds__(K2_MAX_WARPS * 32) k2_ql(const KP<T> p)
     for (int i = 0; i < n; i++) wo[i] = dd[(size_t)i * st];
   }
   p.meta[k] = mt;
-}
-
-// ---------------------------------------------------------------- sorting
-// Permutation of the reference's DO_SORT selection sort (tql2_tiled.hpp:
-// 149-176): for distinct, non-NaN eigenvalues it is the ascending order,
-// computed here by ranks in parallel; with ties or NaNs the serial
-// first-strict-minimum/swap procedure is replayed exactly.
-template <class T>
-__device__ void select_sort_serial(const int n, T *dwork, int *pos)
-{
-  for (int i = 0; i < n; i++) pos[i] = i;
-  for (int l = 0; l < n - 1; l++) {
-    T dl = dwork[l];
-    int il = l;
-    for (int j = l + 1; j < n; j++) {
-      const T dj = dwork[j];
-      if (dl > dj) {
-        dl = dj;
-        il = j;
-      }
-    }
-    if (il != l) {
-      const int t = pos[l];
-      pos[l] = pos[il];
-      pos[il] = t;
-      dwork[il] = dwork[l];
-      dwork[l] = dl;
-    }
-  }
 }
 
 // ---------------------------------------------------------------- phase 3, n <= 32

@@ -190,6 +190,9 @@ template <class T> struct Plan {
   int zsplit = 1;     // phase 3: CTAs per matrix
   int ztm = 0;        // phase 3: rows of Z in tensor memory instead of shared memory
   size_t off_d = 0, off_e = 0, off_meta = 0, off_rec = 0, off_z = 0, bytes = 0;
+  // reflectors of phase 1 (n > 64): in the place of the records, which phase
+  // 2 writes later, unless a caller's rec_cap leaves that too small
+  size_t off_v = 0, vstride = 0;
 };
 
 template <class T> int rec_capacity(int n)
@@ -257,7 +260,10 @@ cudaError_t make_plan(long L, int nm, int n, const DevProps &dp, Plan<T> &pl, co
     }
   }
   const bool zglob = n > 32 && pl.zrows == 0;
-  const size_t per = sizeof(T) * 2 * (size_t)n + sizeof(Meta) + sizeof(Rec<T>) * (size_t)pl.rcap +
+  const size_t rec_b = sizeof(Rec<T>) * (size_t)pl.rcap;
+  const bool vown = n > 64 && (rec_b < fq_bytes<T>(n) || rec_b % 16 != 0);
+  pl.vstride = n > 64 ? (vown ? fq_bytes<T>(n) : rec_b) : 0;
+  const size_t per = sizeof(T) * 2 * (size_t)n + sizeof(Meta) + rec_b + (vown ? pl.vstride : 0) +
                      (zglob ? sizeof(T) * (size_t)n * n : 0);
   long lc = (long)(kWsBudget / per);
   lc = std::max(lc, kMinChunk);
@@ -273,7 +279,9 @@ cudaError_t make_plan(long L, int nm, int n, const DevProps &dp, Plan<T> &pl, co
   pl.off_meta = off;
   off = align256(off + sizeof(Meta) * (size_t)pl.Lc);
   pl.off_rec = off;
-  off = align256(off + sizeof(Rec<T>) * (size_t)pl.rcap * pl.Lc);
+  off = align256(off + rec_b * pl.Lc);
+  pl.off_v = vown ? off : pl.off_rec;
+  if (vown) off = align256(off + pl.vstride * pl.Lc);
   pl.off_z = off;
   if (zglob) off = align256(off + sizeof(T) * (size_t)n * n * pl.Lc);
   pl.bytes = off;
@@ -306,32 +314,140 @@ template <class K> cudaError_t set_smem(K kern, size_t bytes)
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// phase 1 in registers for 32 < n <= 128 (NB = ceil(n/32) column blocks)
-inline int reg_nb(int n) { return (n > 32 && n <= 128) ? (n + 31) / 32 : 0; }
-template <class T> size_t k1r_smem_bytes(int n)
+// phase 1 in registers for 32 < n <= 64 (2 x 2 blocks of 32 x 32).  Above,
+// k1_sym with its separate formation of Q is faster (B200, phase 1 in ms,
+// this form / k1_sym): FP64 n=64 L=20000 4.43 / 5.12, n=96 L=8000 7.68 /
+// 4.35, n=128 L=4096 6.88 / 4.28; FP32 n=64 2.02 / 3.47, n=128 3.34 / 2.65.
+inline bool reg_form(int n) { return n > 32 && n <= 64; }
+template <class T> size_t k1r_smem_bytes(int n) { return sizeof(T) * reg_smem_elems<2>(n); }
+
+// k1_sym: warps, blocks per warp in registers and CTAs per matrix
+struct SymCfg {
+  int nw, rs, cn, mb;  // mb: CTAs an SM the registers are bounded for
+};
+// Measured on B200 (the reduction alone, ms).  Where several matrices fit an
+// SM, small CTAs with few blocks in registers win, their step chains hiding
+// one another: FP64 n=128 L=4096 4 warps x 1 block, three CTAs 3.04, x 2
+// blocks, two CTAs 3.48, 8 x 2, one CTA 5.62; n=160 L=3000 4.65 / 4.05 /
+// 5.69.  From n = 161 on 4 warps no longer have two CTAs an SM (n=192 L=2048
+// 6.58 against 5.20 with 8).  Above 256 the fewest CTAs that hold the
+// triangle: n=512 L=256 4 CTAs 13.4, 8 CTAs 28.8; n=384 L=512 15.3 / 36.8;
+// n=736 L=64 8 CTAs 15.6, 16 CTAs 29.2.  FP32: n=160 L=3000 4 x 1 2.14, 8 x 1
+// 2.80; n=224 L=2048 4.33 / 3.53; n=256 8 x 1 7.06, 4 x 4 5.04, 8 x 4 6.28;
+// n=288 L=1024 4 x 4 5.79, 8 x 4 4.03; n=1000 L=32 8 CTAs 14.2, 16 21.1.
+template <class T> SymCfg sym_cfg(int n)
 {
-  switch (reg_nb(n)) {
-    case 2: return sizeof(T) * reg_smem_elems<2>(n);
-    case 3: return sizeof(T) * reg_smem_elems<3>(n);
-    case 4: return sizeof(T) * reg_smem_elems<4>(n);
-    default: return 0;
+  if (sizeof(T) == 8) {
+    if (n <= 128) return {4, 1, 1, 3};
+    if (n <= 160) return {4, 2, 1, 2};
+    if (n <= 256) return {8, 2, 1, 1};
+    if (n <= 352) return {8, 2, 2, 1};
+    if (n <= 512) return {8, 2, 4, 1};
+    if (n <= 736) return {8, 2, 8, 1};
+    return {8, 2, 16, 1};
+  }
+  if (n <= 160) return {4, 1, 1, 4};
+  if (n <= 224) return {8, 1, 1, 2};
+  if (n <= 256) return {4, 4, 1, 2};
+  if (n <= 384) return {8, 4, 1, 1};
+  if (n <= 512) return {8, 4, 2, 1};
+  if (n <= 736) return {8, 4, 4, 1};
+  return {8, 4, 8, 1};
+}
+template <class T> using SymKernel = void (*)(const KP<T>);
+template <class T> SymKernel<T> sym_kernel(const SymCfg &c)
+{
+  if constexpr (sizeof(T) == 8) {
+    if (c.nw == 4) return c.rs == 1 ? k1_sym<T, 4, 1, 1, 3> : k1_sym<T, 4, 2, 1, 2>;
+    switch (c.cn) {
+      case 1: return k1_sym<T, 8, 2, 1, 1>;
+      case 2: return k1_sym<T, 8, 2, 2, 1>;
+      case 4: return k1_sym<T, 8, 2, 4, 1>;
+      case 8: return k1_sym<T, 8, 2, 8, 1>;
+      default: return k1_sym<T, 8, 2, 16, 1>;
+    }
+  } else {
+    if (c.nw == 4) return c.rs == 1 ? k1_sym<T, 4, 1, 1, 4> : k1_sym<T, 4, 4, 1, 2>;
+    if (c.rs == 1) return k1_sym<T, 8, 1, 1, 2>;
+    switch (c.cn) {
+      case 1: return k1_sym<T, 8, 4, 1, 1>;
+      case 2: return k1_sym<T, 8, 4, 2, 1>;
+      case 4: return k1_sym<T, 8, 4, 4, 1>;
+      default: return k1_sym<T, 8, 4, 8, 1>;
+    }
   }
 }
-template <class T> cudaError_t set_k1r_smem(int n, size_t bytes)
+template <class T> size_t sym_smem(int n, const SymCfg &c)
 {
-  switch (reg_nb(n)) {
-    case 2: return set_smem(k1_reg<T, 2>, bytes);
-    case 3: return set_smem(k1_reg<T, 3>, bytes);
-    case 4: return set_smem(k1_reg<T, 4>, bytes);
-    default: return cudaErrorInvalidValue;
-  }
+  return sizeof(T) * sym_smem_elems(n, c.nw, c.rs, c.cn);
 }
-template <class T> void launch_k1r(const KP<T> &p, unsigned blocks, size_t smem, cudaStream_t st)
+template <class T> cudaLaunchConfig_t sym_launch(int n, const SymCfg &c, long cnt, cudaStream_t st,
+                                                 cudaLaunchAttribute *at)
 {
-  const int nb = reg_nb(p.n);
-  if (nb == 2) k1_reg<T, 2><<<blocks, 32 * 4, smem, st>>>(p);
-  else if (nb == 3) k1_reg<T, 3><<<blocks, 32 * 9, smem, st>>>(p);
-  else k1_reg<T, 4><<<blocks, 32 * 16, smem, st>>>(p);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(cnt * c.cn));
+  cfg.blockDim = dim3(32 * c.nw);
+  cfg.dynamicSmemBytes = sym_smem<T>(n, c);
+  cfg.stream = st;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)c.cn;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = c.cn > 1 ? 1 : 0;
+  return cfg;
+}
+// sets the kernel's attributes and says whether the device can run it (a
+// cluster of 16 needs a GPU processing cluster with that many SMs)
+template <class T> bool sym_usable(int n, const SymCfg &c, const DevProps &dp)
+{
+  const size_t smem = sym_smem<T>(n, c);
+  if (n <= 64 || smem > (size_t)dp.smem_optin) return false;
+  SymKernel<T> kern = sym_kernel<T>(c);
+  if (set_smem(kern, smem) != cudaSuccess) return false;
+  if (c.cn == 1) return true;
+  if (c.cn > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  cudaLaunchAttribute at[1];
+  cudaLaunchConfig_t cfg = sym_launch<T>(n, c, 1, nullptr, at);
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return clusters >= 1;
+}
+
+// formation of Q: column tiles per warp and warps per 8 rows by order
+template <class T> struct FormQ {
+  void (*kern)(const KP<T>, const int);
+  int rows, nbuf;
+  size_t smem;
+};
+template <class T> FormQ<T> form_q_cfg(int n, size_t optin)
+{
+  FormQ<T> f;
+  if (n <= 128) f.kern = k1_formq<T, 16, 1, 2>;
+  else if (n <= 256) f.kern = k1_formq<T, 32, 1, 1>;
+  else if (n <= 512) f.kern = k1_formq<T, 32, 2, 1>;
+  else f.kern = k1_formq<T, 32, 4, 1>;
+  f.rows = fq_rows(n <= 256 ? 1 : (n <= 512 ? 2 : 4));
+  f.nbuf = fq_smem_bytes(n, 2) <= optin ? 2 : 1;
+  f.smem = fq_smem_bytes(n, f.nbuf);
+  return f;
+}
+template <class T> cudaError_t launch_sym(const KP<T> &p, const SymCfg &c, const FormQ<T> &f, long cnt, cudaStream_t st)
+{
+  cudaLaunchAttribute at[1];
+  cudaLaunchConfig_t cfg = sym_launch<T>(p.n, c, cnt, st, at);
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, sym_kernel<T>(c), p);
+  if (err != cudaSuccess) return err;
+  const long warps = cnt * fq_blocks(p.n);
+  k1_factor<T><<<(unsigned)((warps + K1F_NW - 1) / K1F_NW), 32 * K1F_NW, 0, st>>>(p);
+  f.kern<<<(unsigned)(cnt * ((p.n + f.rows - 1) / f.rows)), 256, f.smem, st>>>(p, f.nbuf);
+  return cudaSuccess;
 }
 
 // phase 1 on a cluster: usable when the device can hold one of its
@@ -498,7 +614,10 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
   const int k1c_nt = k1c_threads<T>(n);
   const int red_form = tuned_reduce((int)sizeof(T), n);
   const bool k1_cluster = red_form == EIGEN_GPU_REDUCE_CLUSTER && k1cl_usable<T>(n, dp);
-  const bool k1_in_regs = !k1_cluster && reg_nb(n) > 0 && k1r_smem_bytes<T>(n) <= (size_t)dp.smem_optin;
+  const bool k1_in_regs = !k1_cluster && reg_form(n);
+  const SymCfg k1_symc = sym_cfg<T>(n);
+  const bool k1_symm = !k1_cluster && sym_usable<T>(n, k1_symc, dp);
+  const FormQ<T> k1_fq = form_q_cfg<T>(n, (size_t)dp.smem_optin);
   const size_t k1c_smem = k1_in_regs ? k1r_smem_bytes<T>(n) : sizeof(T) * k1c_smem_elems(n, k1c_nt, pl.k1b);
   size_t k3c_smem = k3c_smem_bytes<T>(n, ztm ? 0 : pl.zrows);
   int k3_wpp = 0, k3_parts = 0, k3_acols = 0;  // tensor-memory form: warps per part, parts per CTA, columns
@@ -579,7 +698,9 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
     if (k1_cluster) {
       // attributes set by k1cl_usable
     } else if (k1_in_regs) {
-      if ((err = set_k1r_smem<T>(n, k1c_smem)) != cudaSuccess) return err;
+      if ((err = set_smem(k1_reg<T, 2>, k1c_smem)) != cudaSuccess) return err;
+    } else if (k1_symm) {  // k1_sym's attributes set by sym_usable
+      if ((err = set_smem(k1_fq.kern, k1_fq.smem)) != cudaSuccess) return err;
     } else if ((err = set_k1_smem<T>(n, k1c_smem)) != cudaSuccess) {
       return err;
     }
@@ -602,7 +723,10 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
       const cudaError_t e = launch_k1cl<T>(q, cnt, st);
       if (e != cudaSuccess && lerr == cudaSuccess) lerr = e;
     } else if (k1_in_regs) {
-      launch_k1r<T>(q, (unsigned)cnt, k1c_smem, st);
+      k1_reg<T, 2><<<(unsigned)cnt, 32 * 4, k1c_smem, st>>>(q);
+    } else if (k1_symm) {
+      const cudaError_t e = launch_sym<T>(q, k1_symc, k1_fq, cnt, st);
+      if (e != cudaSuccess && lerr == cudaSuccess) lerr = e;
     } else {
       launch_k1<T>(q, (unsigned)cnt, k1c_nt, k1c_smem, st);
     }
@@ -635,6 +759,8 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
     p.e = ws_e + wo * n;
     p.meta = ws_meta + wo;
     p.rec = ws_rec + wo * (size_t)pl.rcap;
+    p.vw = reinterpret_cast<unsigned char *>(base) + pl.off_v + wo * pl.vstride;
+    p.vstride = pl.vstride;
     p.zs = ws_z + wo * (size_t)n * n;
     if (ix.kid) {  // the index list advances instead of the pointers
       p.a = a;
@@ -662,9 +788,11 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
   return cudaSuccess;
 }
 
-// Launch geometry of phase 1 (the matrix-parallel reduction) for the first
-// chunk of a default solve, as run() launches it; the counterpart of the
-// reference's eigen_GPU_batch_get_Launch_params (eigen_GPU_batch.hpp:23-102).
+// Launch geometry of the reduction in its one-CTA-per-matrix form (or the
+// cluster form where the tuned options ask for it), for the first chunk of a
+// default solve; the counterpart of the reference's
+// eigen_GPU_batch_get_Launch_params (eigen_GPU_batch.hpp:23-102).  Above
+// n = 64 run() spreads a matrix otherwise (sym_cfg) where the device can.
 template <class T>
 cudaError_t launch_params(long L, int n, int *grp, int *tb, int *gr, int *th, int *sh, int *l2)
 {
@@ -698,12 +826,12 @@ cudaError_t launch_params(long L, int n, int *grp, int *tb, int *gr, int *th, in
     *th = 32 * K1W_NW;
     *tb = (int)((lc + K1W_NW - 1) / K1W_NW);
     *sh = (int)(sizeof(T) * k1w_slot<T>() * K1W_NW);
-  } else if (reg_nb(n) > 0 && k1r_smem_bytes<T>(n) <= (size_t)dp.smem_optin) {  // k1_reg: NB x NB warps
-    const int nb = reg_nb(n);
+  } else if (n <= 128) {  // the register form: NB x NB warps
+    const int nb = (n + 31) / 32;
     *grp = *th = 32 * nb * nb;
     *gr = 1;
     *tb = (int)lc;
-    *sh = (int)k1r_smem_bytes<T>(n);
+    *sh = (int)(sizeof(T) * (nb == 2 ? reg_smem_elems<2>(n) : (nb == 3 ? reg_smem_elems<3>(n) : reg_smem_elems<4>(n))));
   } else {  // k1_cta
     *grp = *th = k1c_threads<T>(n);
     *gr = 1;

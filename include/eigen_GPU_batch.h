@@ -355,7 +355,10 @@ cudaError_t eigen_GPU_batch_symfunc_FP(const int L, const int nm, const int n, c
  * kernel) of a default solve of L matrices of order n on the current
  * device, for the first chunk of the batch; counterpart of the reference's
  * header-only eigen_GPU_batch_get_Launch_params (eigen_GPU_batch.hpp:23-102),
- * which include/eigen_GPU_batch.hpp forwards here.  grpSZ: threads that own
+ * which include/eigen_GPU_batch.hpp forwards here.  The geometry is that of
+ * the one-CTA-per-matrix form in full storage (what a caller who sizes by
+ * threads per matrix wants); above n = 64 the solve itself spreads a matrix
+ * over fewer threads or over a cluster.  grpSZ: threads that own
  * one matrix; numGR: matrices per thread block (1 also for the cluster
  * form, where a matrix spans a cluster of ceil(n/32) blocks and grpSZ
  * counts the cluster's threads); numTH: threads per block; numTB: thread
@@ -390,10 +393,11 @@ typedef struct eigen_GPU_tune_entry {
   int ql_mpw; /* 0: automatic, else a power of two 1..32 */
   int reduce; /* phase-1 kernel: EIGEN_GPU_REDUCE_AUTO, _CTA or _CLUSTER */
 } eigen_GPU_tune_entry;
-/* phase-1 kernels: automatic (the one-CTA forms, measured faster on B200),
- * one CTA per matrix (registers for n <= 128, shared memory and a band in
- * global memory above), or a thread-block cluster holding the matrix in
- * distributed shared memory (32 < n <= 512, where the device can run it).
+/* phase-1 kernels: automatic, which is also what _CTA asks for (one warp or
+ * CTA per matrix while its upper triangle fits one multiprocessor, the
+ * fewest CTAs that hold it above: FP64 n > 256, FP32 n > 384), or a
+ * thread-block cluster holding the whole matrix in distributed shared memory
+ * (32 < n <= 512, where the device can run it; measured slower on B200).
  * Unlike the other entries, the choice changes rounding (another summation
  * order), within the solver's accuracy. */
 #define EIGEN_GPU_REDUCE_AUTO 0
