@@ -16,10 +16,9 @@
 // identity on the wave (its carried value moves on unchanged); the first
 // K-1 steps fill the pipeline and the last K steps drain it.
 //
-// Used by the tensor-memory apply (k3_tmem) for rows of 128 or more; the
-// row accessor below lets the host-side unit tests run the same code on
-// memory.  The shared-memory and workspace forms (k3_cta) keep their
-// pairs of sweeps (seg_apply_pair), measured faster there.
+// This is the pipeline of the wave form of phase 3 (eigb_wave.cuh) as scalar
+// code, for groups of nested sweeps: the host-side unit tests run it against
+// the sweeps one after another.  No kernel calls it.
 #pragma once
 #include "eigb_common.cuh"
 

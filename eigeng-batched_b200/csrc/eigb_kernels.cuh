@@ -19,11 +19,13 @@
 //   k3_warp        phase 3 for n <= 32: rotations applied to Q held in
 //                  registers (one row per lane), selection-sort emulation,
 //                  permuted write-back
-//   k3_cta<SM>     phase 3 for n > 32: rows of Z in shared memory (a
-//                  matrix's rows split over CTAs when needed) or, for the
-//                  largest FP64 sizes, Z in the workspace
-//   k3_tmem        phase 3 for n > 32 with rows of up to 512 32-bit
-//                  columns: rows of Z in tensor memory
+//   k3_tmem        phase 3 for 32 < n < 128: rows of Z in tensor memory
+//   k3_wave        phase 3 for n >= 128: rows of Z in memory, 16 sweeps per
+//                  pass (eigb_wave.cuh)
+//   k3_cta<SM>     phase 3 where the caller asks for shared memory, and for
+//                  n >= 128 the matrices whose records overflowed: rows of Z
+//                  in shared memory (a matrix's rows split over CTAs when
+//                  needed) or, for the largest FP64 sizes, Z in the workspace
 //   k_jacobi_warp  cyclic Jacobi for n <= 32 (jac_tiled.hpp:3-152)
 //   k_check_w      FP64 residual / orthogonality gate (eigen_GPU_check.cu)
 //                  on the FP64 tensor cores, one warp per matrix for
@@ -32,7 +34,7 @@
 #pragma once
 #include <stdio.h>
 
-#include "eigb_apply.cuh"
+#include "eigb_apply.cuh"  // host-tested only
 #include "eigb_common.cuh"
 #include "eigb_formq.cuh"
 #include "eigb_ql.cuh"
@@ -42,6 +44,7 @@
 #include "eigb_tridiag_cl.cuh"
 #include "eigb_tridiag_reg.cuh"
 #include "eigb_tridiag_sym.cuh"
+#include "eigb_wave.cuh"
 
 namespace eigb {
 
@@ -59,6 +62,9 @@ template <class T> struct KP {
   int k1b;       // phase 1 (CTA form): leading block kept in shared memory
   int zrows;     // phase 3 with Z in shared memory: rows per CTA ...
   int zsplit;    // ... and CTAs per matrix
+  int wrows;     // phase 3, wave form: rows per CTA ...
+  int wsplit;    // ... and CTAs per matrix
+  int over;      // phase 3 (CTA form): only the matrices whose records overflowed
   int k2mpw;     // phase 2: matrices per warp (1..32)
   const T *ap;   // packed upper-triangle input (nullptr: the upper triangle of a)
   // uneven batches: matrix k of a launch is matrix kid[k] of the caller's
@@ -507,7 +513,7 @@ __global__ void __launch_bounds__(32 * K3W_NW) k3_warp(const KP<T> p)
 // the other is applied): room for two whole segments.
 // Records per buffer: room for `sweeps` whole sweeps (and their headers),
 // since a sweep is applied only once it is complete in the buffer and a
-// group of sweeps (eigb_apply.cuh) only when all of it is.
+// pair of sweeps only when all of it is.
 __host__ __device__ inline int k3c_chunk(int n, int sweeps = 2) { return ((sweeps * (n + 1) + 63) / 64) * 64; }
 
 template <class T> __host__ __device__ inline size_t k3c_fixed_bytes(int n, int sweeps = 2)
@@ -766,13 +772,12 @@ __device__ __forceinline__ void apply_chunk(const Rec<T> *rbuf, const int used, 
 // column-major, Z(r, c) at Z[r + c*n], so that a warp's accesses at a fixed
 // column are coalesced.
 template <class T, bool SM, int RPT>
-__global__ void __launch_bounds__(SM ? 256 : 512, 1) k3_cta(const KP<T> p)
+__device__ __forceinline__ void k3_cta_part(const KP<T> &p, const long part, unsigned char *smem_raw)
 {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int zsplit = SM ? p.zsplit : 1;
-  const long k = blockIdx.x / zsplit;
+  const long k = part / zsplit;
   const int n = p.n, nm = p.nm, t = threadIdx.x, nt = blockDim.x;
-  const int r0 = SM ? (int)(blockIdx.x % zsplit) * p.zrows : 0;
+  const int r0 = SM ? (int)(part % zsplit) * p.zrows : 0;
   const int nrow = SM ? min(p.zrows, n - r0) : n;
   const int ch = k3c_chunk(n);
   Rec<T> *rbuf = reinterpret_cast<Rec<T> *>(smem_raw);  // two buffers of ch records
@@ -902,17 +907,63 @@ __global__ void __launch_bounds__(SM ? 256 : 512, 1) k3_cta(const KP<T> p)
   }
 }
 
+// One CTA per part, or with p.over a few CTAs that look for the parts of
+// matrices whose records overflowed (none, as a rule).
+template <class T, bool SM, int RPT>
+__global__ void __launch_bounds__(SM ? 256 : 512, 1) k3_cta(const KP<T> p)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const long parts = p.Lc * (long)(SM ? p.zsplit : 1);
+  if (!p.over) {
+    k3_cta_part<T, SM, RPT>(p, blockIdx.x, smem_raw);
+    return;
+  }
+  for (long base = blockIdx.x; base < parts; base += (long)gridDim.x * blockDim.x) {
+    const long mine = base + (long)threadIdx.x * gridDim.x;
+    if (!__syncthreads_or(mine < parts && p.meta[mine / (SM ? p.zsplit : 1)].overflow)) continue;
+    for (long part = base; part < min(parts, base + (long)gridDim.x * blockDim.x); part += gridDim.x)
+      if (p.meta[part / (SM ? p.zsplit : 1)].overflow) {
+        k3_cta_part<T, SM, RPT>(p, part, smem_raw);
+        __syncthreads();
+      }
+  }
+}
+
+// Phase 3, wave form: p.wrows rows of one matrix per CTA, 32 R rows per
+// warp and one more warp that stages the records.  Bound by the latency of the
+// rotation chains between their record loads and by FP64 issue (n=256 FP64:
+// FP64 pipe 52 % active, waits for record loads and for fixed latency 2.6
+// cycles an instruction), so by warps in flight: MB bounds the registers, U
+// the columns in flight that those pay for.  B200, phase 3, ms: FP64 n=256
+// L=2048 two rows per thread, two CTAs an SM and U = 4 14.5, three and U = 2
+// 14.0, one row, four CTAs 16.1; n=144 L=3000 6.93, 6.18, 7.67.
+constexpr int K3W_SWEEPS = 16;
+constexpr int K3W_WARPS = 4;  // row warps per CTA at most
+template <class T, int R, int MB, int U>
+__global__ void __launch_bounds__(32 * (K3W_WARPS + 1), MB) k3_wave(const KP<T> p)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const long k = blockIdx.x / p.wsplit;
+  const int r0 = (int)(blockIdx.x % p.wsplit) * p.wrows;
+  const Meta mt = p.meta[k];
+  if (mt.overflow || r0 >= p.n) return;  // uniform over the CTA
+  wave_apply<T, K3W_SWEEPS, R, U>(mat_ptr(p, k), p.nm, p.n, r0, min(p.wrows, p.n - r0),
+                                  p.rec + (size_t)k * p.rcap, mt.nrec, p.e + k * p.n, p.sort && mt.ierr == 0,
+                                  r0 == 0 ? val_ptr(p, k) : nullptr, smem_raw);
+  if (r0 == 0 && threadIdx.x == 0) put_info(p, k, mt.ierr);
+}
+
 // ---------------------------------------------------------------- phase 3, Z in tensor memory
-// Sweeps per record buffer of k3_tmem: a full group and the next sweep
-// (shared memory is not what limits that kernel).
-constexpr int K3_TM_SWEEPS = K3_GROUP + 1;
+// Sweeps per record buffer of k3_tmem (shared memory is not what limits that
+// kernel).
+constexpr int K3_TM_SWEEPS = 9;
 
 // One part of k3_tmem: rows r0 .. r0+zrows-1 of one matrix, applied by the
 // pn threads pt = 0 .. pn-1 of the part (row r0+pt in tensor memory at z0),
 // with the shared-memory scratch of k3_cta (records double buffer, d, e,
 // sort permutation; no Z) at ps and named barrier id bar.  Same steps and
 // the same arithmetic as k3_cta.
-template <class T, int KG>
+template <class T>
 __device__ __forceinline__ void k3_tmem_part(const KP<T> &p, const long part, const int pt, const int pn,
                                              const int bar, unsigned char *ps, const uint32_t z0)
 {
@@ -968,7 +1019,7 @@ __device__ __forceinline__ void k3_tmem_part(const KP<T> &p, const long part, co
         for (int q = pt; q < ncnt; q += pn) cp_async<sizeof(Rec<T>)>(nx + q, src + nb + q);
         cp_async_commit();
       }
-      apply_segments_tm<T, KG>(rb, used, z0);
+      apply_segments_tm<T>(rb, used, z0);
       cp_async_wait_all();
       part_sync(bar, pn);
       base = nb;
@@ -995,7 +1046,7 @@ __device__ __forceinline__ void k3_tmem_part(const KP<T> &p, const long part, co
       part_sync(bar, pn);
       const int nr = sflag[0];
       const int done = sflag[1];
-      apply_segments_tm<T, KG>(rbuf, nr, z0);
+      apply_segments_tm<T>(rbuf, nr, z0);
       part_sync(bar, pn);
       if (done) break;
     }
@@ -1056,7 +1107,7 @@ __device__ __forceinline__ void k3_tmem_part(const KP<T> &p, const long part, co
 // 32*(w % 4) .., in the acols columns the CTA allocates.  The host sizes
 // the CTA's shared memory in proportion to acols, so the CTAs that share an
 // SM never hold more than its 512 columns together.
-template <class T, int KG>
+template <class T>
 __global__ void __launch_bounds__(128, 1) k3_tmem(const KP<T> p, const int wpp, const int acols)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1072,7 +1123,7 @@ __global__ void __launch_bounds__(128, 1) k3_tmem(const KP<T> p, const int wpp, 
   tmem_fence_after();
   const uint32_t z0 = tbase + ((uint32_t)(32 * (w & 3)) << 16);
   if (part < p.Lc * (long)p.zsplit)  // uniform per part
-    k3_tmem_part<T, KG>(p, part, t - g * pn, pn, parts == 1 ? 0 : 1 + g,
+    k3_tmem_part<T>(p, part, t - g * pn, pn, parts == 1 ? 0 : 1 + g,
                     smem_raw + (size_t)g * k3c_fixed_bytes<T>(p.n, K3_TM_SWEEPS), z0);
   // every tensor memory access of the CTA is complete (loads wait in
   // place, stores before the read-out); the allocating warp frees

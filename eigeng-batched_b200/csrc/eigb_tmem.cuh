@@ -22,7 +22,6 @@
 #pragma once
 #include <stdint.h>
 
-#include "eigb_apply.cuh"
 #include "eigb_common.cuh"
 
 namespace eigb {
@@ -240,15 +239,6 @@ __device__ __forceinline__ void seg_apply_tm(const uint32_t z0, const Rec<T> *__
   seg_apply_tm_h<T>(z0, rp, i0, len, tmem_ld1((const T *)nullptr, tmem_at<T>(z0, i0 + 1)));
 }
 
-// Row accessor for seg_apply_group: this thread's row in TMEM
-template <class T> struct RowTM {
-  uint32_t z0;
-  __device__ __forceinline__ T ld(const int c) const { return tmem_ld1((const T *)nullptr, tmem_at<T>(z0, c)); }
-  __device__ __forceinline__ void st(const int c, const T v) const { tmem_st1(tmem_at<T>(z0, c), v); }
-  __device__ __forceinline__ void ld8(const int c, T (&v)[8]) const { tmem_ld8(tmem_at<T>(z0, c), v); }
-  __device__ __forceinline__ void begin() const { tmem_wait_st(); }  // earlier stores land before these loads
-};
-
 // seg_apply_pair on a row in TMEM (bit-identical to the shared-memory form)
 template <class T>
 __device__ __forceinline__ void seg_apply_pair_tm(const uint32_t z0, const Rec<T> *__restrict__ ra, const int la,
@@ -303,27 +293,12 @@ __device__ __forceinline__ void seg_apply_pair_tm(const uint32_t z0, const Rec<T
   }
 }
 
-// A single sweep on a row in TMEM (functor for apply_grouped)
-template <class T> struct SingleTM {
-  uint32_t z0;
-  __device__ __forceinline__ void operator()(const Rec<T> *rp, const int i0, const int len) const
-  {
-    seg_apply_tm<T>(z0, rp, i0, len);
-  }
-};
-
 // apply_segments for a row in TMEM (bit-identical to the shared-memory
-// form).  KG > 1: groups of up to KG consecutive sweeps go through
-// seg_apply_group; KG = 1: two consecutive sweeps from the same top, the
-// second no longer than the first, go through seg_apply_pair_tm (measured on B200: groups pay off for rows
-// of 128 or more, the pairs below that).
-template <class T, int KG>
+// form): two consecutive sweeps from the same top, the second no longer than
+// the first, go through seg_apply_pair_tm.
+template <class T>
 __device__ __forceinline__ void apply_segments_tm(const Rec<T> *rbuf, const int used, const uint32_t z0)
 {
-  if (KG > 1) {
-    apply_grouped<T, KG>(rbuf, used, RowTM<T>{z0}, SingleTM<T>{z0});
-    return;
-  }
   int q = 0;
   while (q < used) {
     const Rec<T> hd = rbuf[q];

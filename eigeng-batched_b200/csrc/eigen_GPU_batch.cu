@@ -238,7 +238,9 @@ cudaError_t make_plan(long L, int nm, int n, const DevProps &dp, Plan<T> &pl, co
     // on B200: FP64 n = 160, two parts of 80 rows with one CTA per SM, is
     // slower than one shared-memory CTA of 160 rows; FP32 n = 200, two
     // parts of 100 rows with two CTAs per SM, is faster than one of 200)
-    if (pl.zrows > 0 && tmem_cols<T>(n) > 0 && !(opts && opts->zmem == EIGEN_GPU_ZMEM_SHARED)) {
+    // From n = 128 on the wave form is faster and the plan here serves the
+    // matrices it leaves out.
+    if (n < 128 && pl.zrows > 0 && tmem_cols<T>(n) > 0 && !(opts && opts->zmem == EIGEN_GPU_ZMEM_SHARED)) {
       int split = (n + 127) / 128;
       const int want = opts ? opts->split : 0;
       if (want > split) split = std::min(want, (n + 31) / 32);
@@ -310,7 +312,7 @@ cudaError_t buffer_size(long L, int nm, int n, int m, size_t *lwork, const eigen
 
 template <class K> cudaError_t set_smem(K kern, size_t bytes)
 {
-  if (bytes <= 48 * 1024) return cudaSuccess;
+  if (bytes <= 46 * 1024) return cudaSuccess;  // 48 KB less the static shared memory of any kernel here
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
@@ -621,14 +623,7 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
   const size_t k1c_smem = k1_in_regs ? k1r_smem_bytes<T>(n) : sizeof(T) * k1c_smem_elems(n, k1c_nt, pl.k1b);
   size_t k3c_smem = k3c_smem_bytes<T>(n, ztm ? 0 : pl.zrows);
   int k3_wpp = 0, k3_parts = 0, k3_acols = 0;  // tensor-memory form: warps per part, parts per CTA, columns
-  // sweeps per pass: up to eight for rows of 256 or more, four for rows of
-  // 128 .. 255, pairs below 128 (measured on B200: the longer groups give
-  // each thread more independent rotation chains, at 254 registers, which
-  // costs the CTAs that share an SM; at FP64 n=128 eight save 0.12 ms of
-  // phase 3 alone but lose 1.7 ms of a host-to-host solve, where the other
-  // chunks' phase-1/2 CTAs run beside phase 3)
-  void (*k3t)(const KP<T>, const int, const int) =
-      n < 128 ? k3_tmem<T, 1> : (n >= 256 ? k3_tmem<T, 8> : k3_tmem<T, 4>);
+  void (*k3t)(const KP<T>, const int, const int) = k3_tmem<T>;
   if (ztm) {
     // Tensor memory is allocated per CTA, and the CTAs on one SM must never
     // ask for more than its 512 columns together (an allocation would wait
@@ -669,6 +664,34 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
     }
   }
   const bool zsm = pl.zrows > 0 && !ztm;
+  // Wave form of phase 3 from n = 128 on, unless the caller asks for Z in
+  // shared memory.  Up to 256 rows per CTA, two rows per thread; one where
+  // that leaves an SM fewer than four warps, or where the rows of a matrix
+  // are four warps at one row each.  Measured on B200 (phase 3, ms, former
+  // form / this): FP64 n=128 L=4096 3.71 / 3.63 (two rows 3.73), n=200 L=2048
+  // 14.6 / 8.9, n=256 22.2 / 14.0, n=512 L=256 58.5 / 14.9, n=1000 L=32 163 /
+  // 17.2 (two rows 19.1); FP32 n=128 L=4096 1.77 / 1.90, n=201 L=1000 2.88 /
+  // 2.26, n=256 L=2048 8.30 / 6.72.  Below 128 the fill and drain of 16 sweeps
+  // weigh too much: FP64 n=64 L=20000 2.79 / 5.13.
+  const bool wave = n >= 128 && !(opts && opts->zmem == EIGEN_GPU_ZMEM_SHARED);
+  constexpr int WMB = sizeof(T) == 8 ? 3 : 2, WU = sizeof(T) == 8 ? 2 : 4;
+  void (*kwave)(const KP<T>) = k3_wave<T, 2, WMB, WU>;
+  unsigned wave_nt = 0;
+  const size_t wave_smem = wv_smem_bytes<T>(n, K3W_SWEEPS);
+  if (wave) {
+    const bool few = std::min(count, pl.Lc) * ((n + 63) / 64) < 4L * dp.sms;
+    int rw = 64;
+    if (few || (sizeof(T) == 8 && n <= 32 * K3W_WARPS)) {
+      rw = 32;
+      kwave = few ? k3_wave<T, 1, 2, 4> : k3_wave<T, 1, 4, 4>;
+    }
+    p.wsplit = (n + rw * K3W_WARPS - 1) / (rw * K3W_WARPS);
+    const int want = opts ? opts->split : 0;
+    if (want > p.wsplit) p.wsplit = std::min(want, (n + 31) / 32);
+    p.wrows = (n + p.wsplit - 1) / p.wsplit;
+    wave_nt = 32u * ((p.wrows + rw - 1) / rw + 1);
+    if ((err = set_smem(kwave, wave_smem)) != cudaSuccess) return err;
+  }
   // phase 2: matrices per warp, then warps per block within the shared
   // memory budget (2n values per matrix)
   p.k2mpw = k2_mpw(std::min(count, pl.Lc), dp.sms);
@@ -741,12 +764,18 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
       const long nparts = cnt * pl.zsplit;
       k3t<<<(unsigned)((nparts + k3_parts - 1) / k3_parts), 32 * k3_wpp * k3_parts, k3c_smem, st>>>(
           q, k3_wpp, k3_acols);
-    } else if (zsm) {
-      k3_cta<T, true, 1><<<(unsigned)(cnt * pl.zsplit), k3_nt, k3c_smem, st>>>(q);
-    } else if (n > 512) {
-      k3_cta<T, false, 2><<<(unsigned)cnt, k3_nt, k3c_smem, st>>>(q);
     } else {
-      k3_cta<T, false, 1><<<(unsigned)cnt, k3_nt, k3c_smem, st>>>(q);
+      KP<T> o = q;
+      long blocks = cnt * (zsm ? pl.zsplit : 1);
+      if (wave) {
+        const unsigned wb = (unsigned)(cnt * q.wsplit);
+        kwave<<<wb, wave_nt, wave_smem, st>>>(q);
+        o.over = 1;
+        blocks = std::min<long>(blocks, dp.sms);
+      }
+      if (zsm) k3_cta<T, true, 1><<<(unsigned)blocks, k3_nt, k3c_smem, st>>>(o);
+      else if (n > 512) k3_cta<T, false, 2><<<(unsigned)blocks, k3_nt, k3c_smem, st>>>(o);
+      else k3_cta<T, false, 1><<<(unsigned)blocks, k3_nt, k3c_smem, st>>>(o);
     }
   };
   for (long c0 = first; c0 < first + count; c0 += pl.Lc) {
