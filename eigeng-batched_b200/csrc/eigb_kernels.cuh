@@ -331,18 +331,15 @@ __global__ void __launch_bounds__(K2_MAX_WARPS * 32) k2_ql(const KP<T> p)
   const long k = (long)blockIdx.x * st + slot;
   if (k >= p.Lc) return;
   const int n = p.n;
-  T *dd = reinterpret_cast<T *>(smem_raw) + slot;
-  T *ee = dd + (size_t)n * st;
+  using V = typename DEVec<T>::V;
+  const DEPair<T> de{reinterpret_cast<V *>(smem_raw) + slot, st};
   const T *din = p.d + k * n;
   const T *ein = p.e + k * n;
-  for (int i = 0; i < n; i++) {
-    dd[(size_t)i * st] = din[i];
-    ee[(size_t)i * st] = ein[i];
-  }
+  for (int i = 0; i < n; i++) de.put(de.at(i), 0, din[i], ein[i]);
   Rec<T> *out = p.rec + (size_t)k * p.rcap;
   int ierr = 0;
-  const int nr = (p.method == QL_IMTQL2) ? ql_imtql2_fast(dd, ee, st, n, out, p.rcap, p.max_sweep, &ierr)
-                                         : ql_tql2_fast(dd, ee, st, n, out, p.rcap, p.max_sweep, &ierr);
+  const int nr = (p.method == QL_IMTQL2) ? ql_imtql2_fast_s<T>(de, n, out, p.rcap, p.max_sweep, &ierr)
+                                         : ql_tql2_fast_s<T>(de, n, out, p.rcap, p.max_sweep, &ierr);
   Meta mt;
   mt.nrec = nr < 0 ? 0 : nr;
   mt.pad = 0;
@@ -355,7 +352,7 @@ __global__ void __launch_bounds__(K2_MAX_WARPS * 32) k2_ql(const KP<T> p)
     // unsorted eigenvalues over e (no longer needed): phase 3 reads them
     // from there in every CTA of the matrix, and writes w sorted
     T *wo = p.e + k * n;
-    for (int i = 0; i < n; i++) wo[i] = dd[(size_t)i * st];
+    for (int i = 0; i < n; i++) wo[i] = de.d(de.at(i), 0);
   }
   p.meta[k] = mt;
 }

@@ -42,17 +42,49 @@ template <class T> struct DEView {
 // One tql2 chase step at index i (tql2_tiled.hpp:94-115): from the
 // previous (c, s, p) and (e_i, d_i) to the new rotation (cn, sn), the new p
 // and the values stored at i+1.  Shared by both generators.
+//
+// The next step waits for pn alone, so that is formed as y q with q = p d_i
+// - c e_i^2 ready before y = 1/sqrt(p^2 + e_i^2).
+template <class T> struct Tql2Step {
+  T cn, sn, r, pn, gg, h;
+};
+template <class T> struct Tql2Pre {
+  T sig, y, q, gg, h;
+};
+// what the step needs before its rotation, y on its way ...
 template <class T>
-__host__ __device__ __forceinline__ void tql2_step(const T c, const T s, const T p, const T ei, const T di, T &cn,
-                                                   T &sn, T &pn, T &ei1, T &di1)
+__host__ __device__ __forceinline__ Tql2Pre<T> tql2_begin(const T c, const T p, const T ei, const T di)
 {
-  const T gg = mul_rn(c, ei);
-  const T h = mul_rn(c, p);
-  T r;
-  givens(p, ei, cn, sn, r);
-  ei1 = mul_rn(s, r);
-  pn = fma(cn, di, -mul_rn(sn, gg));
-  di1 = fma(sn, fma(cn, gg, mul_rn(sn, di)), h);
+  Tql2Pre<T> a;
+  a.sig = fma(p, p, mul_rn(ei, ei));
+  a.gg = mul_rn(c, ei);
+  a.h = mul_rn(c, p);
+  a.q = fma(p, di, -mul_rn(ei, a.gg));
+  a.y = rsq_fast(a.sig);
+  return a;
+}
+// ... and the rotation
+template <class T>
+__host__ __device__ __forceinline__ Tql2Step<T> tql2_end(const Tql2Pre<T> &a, const T p, const T ei, const T di)
+{
+  Tql2Step<T> k;
+  k.gg = a.gg;
+  k.h = a.h;
+  k.cn = mul_rn(p, a.y);
+  k.sn = mul_rn(ei, a.y);
+  k.r = mul_rn(a.sig, a.y);
+  k.pn = mul_rn(a.y, a.q);
+  if (!rsq_plain(a.sig)) {
+    givens_any(p, ei, k.cn, k.sn, k.r);
+    k.pn = fma(k.cn, di, -mul_rn(k.sn, k.gg));
+  }
+  return k;
+}
+// the values stored at i+1, from the step's rotation and the s before it
+template <class T> __host__ __device__ __forceinline__ T tql2_e1(const Tql2Step<T> &k, const T s) { return mul_rn(s, k.r); }
+template <class T> __host__ __device__ __forceinline__ T tql2_d1(const Tql2Step<T> &k, const T di)
+{
+  return fma(k.sn, fma(k.cn, k.gg, mul_rn(k.sn, di)), k.h);
 }
 
 // Explicit shift of tql2 (tql2_tiled.hpp:64-75): new d(l), d(l+1).
@@ -179,17 +211,16 @@ __host__ __device__ int ql_tql2(QLGen<T> &g, const DEView<T> v, const int n, Rec
             g.s2 = g.s;
             const T ei = v.E(i);
             const T di = (i >= g.l + 2) ? v.D(i) - g.delta : v.D(i);
-            T c, s, pn, ei1, di1;
-            tql2_step(g.c, g.s, g.p, ei, di, c, s, pn, ei1, di1);
-            g.p = pn;
-            v.E(i + 1) = ei1;
-            v.D(i + 1) = di1;
-            g.c = c;
-            g.s = s;
+            const Tql2Step<T> k = tql2_end(tql2_begin(g.c, g.p, ei, di), g.p, ei, di);
+            g.p = k.pn;
+            v.E(i + 1) = tql2_e1(k, g.s);
+            v.D(i + 1) = tql2_d1(k, di);
+            g.c = k.cn;
+            g.s = k.sn;
             g.ei = ei;
             Rec<T> rec;
-            rec.c = c;
-            rec.s = s;
+            rec.c = k.cn;
+            rec.s = k.sn;
             buf[nrec++] = rec;
             g.seg_cnt++;
           }
@@ -308,26 +339,108 @@ finish:
 // rotations and eigenvalues).  Returns the record count, or -1 when the
 // capacity would be exceeded (phase 3 then regenerates with the resumable
 // form).  *ierr receives 0 or the failing 1-based index.
-template <class T>
-__host__ __device__ int ql_tql2_fast(T *__restrict__ d, T *__restrict__ e, const int st, const int n,
-                                     Rec<T> *__restrict__ out, const int cap, const int max_sweep, int *ierr)
+//
+// Storage of a chain: element i of d and e at stride st, in two arrays
+// (DESep) or, on the GPU, as pairs, one load and one store for both (DEPair).
+template <class T> struct DESep {
+  T *dp, *ep;
+  int st;
+  struct Cur {
+    T *d, *e;
+  };
+  __host__ __device__ __forceinline__ Cur at(int i) const { return Cur{dp + i * st, ep + i * st}; }
+  __host__ __device__ __forceinline__ void move(Cur &c, int k) const
+  {
+    c.d += k * st;
+    c.e += k * st;
+  }
+  __host__ __device__ __forceinline__ T d(const Cur &c, int k) const { return c.d[k * st]; }
+  __host__ __device__ __forceinline__ T e(const Cur &c, int k) const { return c.e[k * st]; }
+  __host__ __device__ __forceinline__ void get(const Cur &c, int k, T &x, T &y) const
+  {
+    x = c.d[k * st];
+    y = c.e[k * st];
+  }
+  __host__ __device__ __forceinline__ void put(const Cur &c, int k, T x, T y) const
+  {
+    c.d[k * st] = x;
+    c.e[k * st] = y;
+  }
+  __host__ __device__ __forceinline__ void put_d(const Cur &c, int k, T x) const { c.d[k * st] = x; }
+  __host__ __device__ __forceinline__ void put_e(const Cur &c, int k, T y) const { c.e[k * st] = y; }
+};
+template <class T> struct DEVec;
+template <> struct DEVec<double> { using V = double2; };
+template <> struct DEVec<float> { using V = float2; };
+template <class T> struct DEPair {
+  using V = typename DEVec<T>::V;
+  V *q;
+  int st;
+  using Cur = V *;
+  __host__ __device__ __forceinline__ Cur at(int i) const { return q + i * st; }
+  __host__ __device__ __forceinline__ void move(Cur &c, int k) const { c += k * st; }
+  __host__ __device__ __forceinline__ T d(const Cur &c, int k) const { return c[k * st].x; }
+  __host__ __device__ __forceinline__ T e(const Cur &c, int k) const { return c[k * st].y; }
+  __host__ __device__ __forceinline__ void get(const Cur &c, int k, T &x, T &y) const
+  {
+    const V v = c[k * st];
+    x = v.x;
+    y = v.y;
+  }
+  __host__ __device__ __forceinline__ void put(const Cur &c, int k, T x, T y) const
+  {
+    V v;
+    v.x = x;
+    v.y = y;
+    c[k * st] = v;
+  }
+  __host__ __device__ __forceinline__ void put_d(const Cur &c, int k, T x) const { c[k * st].x = x; }
+  __host__ __device__ __forceinline__ void put_e(const Cur &c, int k, T y) const { c[k * st].y = y; }
+};
+
+// The rotation loop is bound by the latency of its recurrence (p -> y -> p)
+// and, with several chains a scheduler, by instruction issue.  What a
+// rotation leaves behind (its record, d and e of i+1) is therefore formed and
+// stored one step later, while that step's y is on its way, in one block
+// without branches but for rsq_plain's, and four steps are unrolled, which
+// turns the hand-over from step to step into register names.  Measured on
+// B200 against the loop that finished each rotation in place with the
+// library's rsqrt (phase 2, ms; not unrolled in brackets): FP64 n=128 L=4096
+// 2.44 -> 1.59 (1.80), n=256 L=2048 10.7 -> 6.4 (7.4), n=512 L=256 30.0 ->
+// 18.5 (21.2), n=1000 L=32 109 -> 67 (77); FP32 n=128 2.36 -> 1.11 (1.27),
+// n=256 9.2 -> 4.3 (5.0).
+template <class T, class S>
+__host__ __device__ int ql_tql2_fast_s(const S v, const int n, Rec<T> *__restrict__ out, const int cap,
+                                       const int max_sweep, int *ierr)
 {
+  using Cur = typename S::Cur;
   const T tol = Num<T>::eps() * Num<T>::tolmul();
   int nrec = 0;
   *ierr = 0;
   if (n <= 1) return 0;
   T shift = T(0), tst1 = T(0);
   for (int l = 0; l < n; l++) {
-    T *dl_p = d + l * st;
-    T *el_p = e + l * st;
-    tst1 = fmax_t(tst1, (fabs_t(*dl_p) + fabs_t(*el_p)) * tol);
-    int m = l;
+    const Cur lp = v.at(l);
     {
-      const T *ep = el_p;
-      while (m < n && !(fabs_t(*ep) <= tst1)) {
-        m++;
-        ep += st;
+      T d0, e0;
+      v.get(lp, 0, d0, e0);
+      tst1 = fmax_t(tst1, (fabs_t(d0) + fabs_t(e0)) * tol);
+    }
+    int m = l;
+    {  // first m >= l with |e(m)| <= tst1, four at a time
+      Cur ep = lp;
+      bool found = false;
+      for (; m + 4 <= n; m += 4, v.move(ep, 4)) {
+        const T a0 = v.e(ep, 0), a1 = v.e(ep, 1), a2 = v.e(ep, 2), a3 = v.e(ep, 3);
+        const bool b0 = fabs_t(a0) <= tst1, b1 = fabs_t(a1) <= tst1, b2 = fabs_t(a2) <= tst1, b3 = fabs_t(a3) <= tst1;
+        if (b0 || b1 || b2 || b3) {
+          m += b0 ? 0 : (b1 ? 1 : (b2 ? 2 : 3));
+          found = true;
+          break;
+        }
       }
+      if (!found)
+        for (; m < n && !(fabs_t(v.e(ep, 0)) <= tst1); m++) v.move(ep, 1);
     }
     if (m >= n) {
       *ierr = l + 1;
@@ -338,71 +451,81 @@ __host__ __device__ int ql_tql2_fast(T *__restrict__ d, T *__restrict__ e, const
       int itr;
       for (itr = 0; itr < max_sweep; itr++) {
         if (nrec + 1 + len > cap) return -1;
-        const T dl_old = *dl_p;
-        T dl, dl1;
-        tql2_shift(dl_old, dl_p[st], *el_p, dl, dl1);
-        *dl_p = dl;
-        dl_p[st] = dl1;
+        T dl_old, el, dl1_old, el1, dl, dl1;
+        v.get(lp, 0, dl_old, el);
+        v.get(lp, 1, dl1_old, el1);
+        tql2_shift(dl_old, dl1_old, el, dl, dl1);
+        v.put_d(lp, 0, dl);
+        v.put_d(lp, 1, dl1);
         const T delta = dl_old - dl;
-        for (int j = m + 1; j < n; j++) d[j * st] -= delta;  // d(l+2..m) are shifted on read
+        {  // d(l+2..m) are shifted on read
+          Cur jp = v.at(m + 1);
+          for (int j = m + 1; j < n; j++, v.move(jp, 1)) v.put_d(jp, 0, v.d(jp, 0) - delta);
+        }
         shift += delta;
         T c = T(1), c2 = T(1), c3 = T(1), s = T(0), s2 = T(0);
-        T *dp = d + m * st;
-        T *ep = e + (m - 1) * st;
-        T p = (m >= l + 2) ? *dp - delta : *dp;
-        const T el1 = el_p[st];
-        T ei = T(0);
-        Rec<T> *o = out + nrec + 1;
-        // e(i), d(i) of the next step are loaded before this step's stores
-        // of e(i+1), d(i+1) (distinct addresses)
-        T ei_n = *ep, dsi_n = dp[-st];
+        Cur qp = v.at(m);  // i+1
+        T p = (m >= l + 2) ? v.d(qp, 0) - delta : v.d(qp, 0);
+        T ei = T(0), di = T(0), so = T(0);
+        // the step whose outputs are pending; its record goes to *o, the
+        // segment's header slot (written last) while there is none
+        Tql2Step<T> k;
+        k.cn = k.sn = k.r = k.pn = k.gg = k.h = T(0);
+        Rec<T> *o = out + nrec;
+        T d_n, e_n;  // the next step's d(i), e(i), loaded a step ahead
+        v.get(qp, -1, d_n, e_n);
+#pragma unroll 4
         for (int i = m - 1; i >= l; i--) {
           c3 = c2;
           c2 = c;
           s2 = s;
-          ei = ei_n;
-          const T dsi = dsi_n;
-          if (i > l) {
-            ei_n = ep[-st];
-            dsi_n = dp[-2 * st];
-          }
-          const T di = (i >= l + 2) ? dsi - delta : dsi;
-          T cn, sn, pn, ei1, di1;
-          tql2_step(c, s, p, ei, di, cn, sn, pn, ei1, di1);
-          ep[st] = ei1;
-          p = pn;
-          *dp = di1;
-          c = cn;
-          s = sn;
+          ei = e_n;
+          const T dn = (i >= l + 2) ? d_n - delta : d_n;
+          v.get(qp, i > l ? -2 : -1, d_n, e_n);
+          const Tql2Pre<T> a = tql2_begin(c, p, ei, dn);
+          const T e1 = tql2_e1(k, so), d1 = tql2_d1(k, di);
           Rec<T> rec;
-          rec.c = cn;
-          rec.s = sn;
+          rec.c = c;
+          rec.s = s;
           *o++ = rec;
-          dp -= st;
-          ep -= st;
+          if (i < m - 1) v.put(qp, 1, d1, e1);
+          k = tql2_end(a, p, ei, dn);
+          di = dn;
+          so = s;
+          p = k.pn;
+          c = k.cn;
+          s = k.sn;
+          v.move(qp, -1);
+        }
+        v.put(qp, 1, tql2_d1(k, di), tql2_e1(k, so));
+        {
+          Rec<T> rec;
+          rec.c = c;
+          rec.s = s;
+          *o = rec;
         }
         out[nrec] = make_hdr(m - 1, len, T(0));
         nrec += 1 + len;
         T eln, dln;
         tql2_close(c, s, s2, c3, el1, ei, dl1, eln, dln);
-        *el_p = eln;
-        *dl_p = dln;
-        if (fabs_t(*el_p) <= tst1) break;
+        v.put(lp, 0, dln, eln);
+        if (fabs_t(eln) <= tst1) break;
       }
       if (itr >= max_sweep) {
         *ierr = l + 1;
         return nrec;
       }
     }
-    *dl_p += shift;
+    v.put_d(lp, 0, v.d(lp, 0) + shift);
   }
   return nrec;
 }
 
-template <class T>
-__host__ __device__ int ql_imtql2_fast(T *__restrict__ d, T *__restrict__ e, const int st, const int n,
-                                       Rec<T> *__restrict__ out, const int cap, const int max_sweep, int *ierr)
+template <class T, class S>
+__host__ __device__ int ql_imtql2_fast_s(const S v, const int n, Rec<T> *__restrict__ out, const int cap,
+                                         const int max_sweep, int *ierr)
 {
+  using Cur = typename S::Cur;
   const T tol = Num<T>::eps() * Num<T>::tolmul();
   int nrec = 0;
   *ierr = 0;
@@ -411,23 +534,31 @@ __host__ __device__ int ql_imtql2_fast(T *__restrict__ d, T *__restrict__ e, con
     int itr;
     for (itr = 0; itr <= max_sweep; itr++) {
       int m = n - 1;
-      for (int mm = l; mm < n - 1; mm++) {
-        const T t1 = (fabs_t(d[mm * st]) + fabs_t(d[(mm + 1) * st])) * tol;
-        if (!(fabs_t(e[mm * st]) > t1)) {
-          m = mm;
-          break;
+      {
+        Cur mp = v.at(l);
+        T d0, e0;
+        for (int mm = l; mm < n - 1; mm++, v.move(mp, 1)) {
+          v.get(mp, 0, d0, e0);
+          const T t1 = (fabs_t(d0) + fabs_t(v.d(mp, 1))) * tol;
+          if (!(fabs_t(e0) > t1)) {
+            m = mm;
+            break;
+          }
         }
       }
       if (m == l) break;
       if (nrec + 1 + (m - l) > cap) return -1;
-      T di1 = d[m * st];
-      T r = imtql2_shift(d[l * st], d[(l + 1) * st], e[l * st], di1);
+      const Cur lp = v.at(l);
+      Cur ip = v.at(m);  // i+1
+      T di1 = v.d(ip, 0);
+      T r = imtql2_shift(v.d(lp, 0), v.d(lp, 1), v.e(lp, 0), di1);
       T s = T(1), c = T(1), delta = T(0);
       Rec<T> *o = out + nrec + 1;
       int i;
       int cnt = 0;
       for (i = m - 1; i >= l; i--) {
-        const T ei = e[i * st];
+        T di, ei;
+        v.get(ip, -1, di, ei);
         const T f = mul_rn(s, ei);
         T cn, sn, rn;
         givens(r, f, cn, sn, rn);
@@ -435,9 +566,8 @@ __host__ __device__ int ql_imtql2_fast(T *__restrict__ d, T *__restrict__ e, con
           r = T(0);
           break;
         }
-        const T dx1 = imtql2_step(cn, sn, c, ei, d[i * st], di1, delta, r);
-        e[(i + 1) * st] = rn;
-        d[(i + 1) * st] = dx1;
+        const T dx1 = imtql2_step(cn, sn, c, ei, di, di1, delta, r);
+        v.put(ip, 0, dx1, rn);
         c = cn;
         s = sn;
         Rec<T> rec;
@@ -445,15 +575,15 @@ __host__ __device__ int ql_imtql2_fast(T *__restrict__ d, T *__restrict__ e, con
         rec.s = sn;
         *o++ = rec;
         cnt++;
+        v.move(ip, -1);
       }
       if (cnt > 0) {
         out[nrec] = make_hdr(m - 1, cnt, T(0));
         nrec += 1 + cnt;
       }
-      const int j = (i + 1 > l) ? i + 1 : l;
-      d[j * st] -= delta;
-      e[j * st] = r;
-      e[m * st] = T(0);
+      const Cur jp = v.at((i + 1 > l) ? i + 1 : l);
+      v.put(jp, 0, v.d(jp, 0) - delta, r);
+      v.put_e(v.at(m), 0, T(0));
     }
     if (itr > max_sweep) {
       *ierr = l + 1;
@@ -464,7 +594,23 @@ __host__ __device__ int ql_imtql2_fast(T *__restrict__ d, T *__restrict__ e, con
 }
 
 template <class T>
-__host__ __device__ __forceinline__ int ql_run(int method, QLGen<T> &g, const DEView<T> v, const int n,
+__host__ __device__ int ql_tql2_fast(T *__restrict__ d, T *__restrict__ e, const int st, const int n,
+                                     Rec<T> *__restrict__ out, const int cap, const int max_sweep, int *ierr)
+{
+  return ql_tql2_fast_s<T>(DESep<T>{d, e, st}, n, out, cap, max_sweep, ierr);
+}
+template <class T>
+__host__ __device__ int ql_imtql2_fast(T *__restrict__ d, T *__restrict__ e, const int st, const int n,
+                                       Rec<T> *__restrict__ out, const int cap, const int max_sweep, int *ierr)
+{
+  return ql_imtql2_fast_s<T>(DESep<T>{d, e, st}, n, out, cap, max_sweep, ierr);
+}
+
+// Not inlined: it runs for the rare matrix whose records overflowed, and its
+// state would cost the apply kernels registers (k3_warp n=32 L=16384: 0.60 ms,
+// inlined 0.80).
+template <class T>
+__host__ __device__ __noinline__ int ql_run(int method, QLGen<T> &g, const DEView<T> v, const int n,
                                       Rec<T> *buf, const int cap, const int max_sweep)
 {
   return method == QL_IMTQL2 ? ql_imtql2(g, v, n, buf, cap, max_sweep)

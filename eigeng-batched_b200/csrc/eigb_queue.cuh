@@ -8,7 +8,7 @@
 // queue, an atomic counter over a job list sorted by decreasing order
 // (longest processing time first: the longest chains start at once, the
 // short ones fill in behind them).  Each job runs the same recurrence as
-// k2_ql (ql_tql2_fast / ql_imtql2_fast on a shared-memory copy of d and e:
+// k2_ql (ql_tql2_fast_s / ql_imtql2_fast_s on a shared-memory copy of d and e:
 // identical rotations and eigenvalues) and leaves the records, the status
 // block and the unsorted eigenvalues exactly where k2_ql leaves them, so the
 // apply phase of each group runs unchanged.
@@ -42,8 +42,8 @@ __global__ void __launch_bounds__(K2_MAX_WARPS * 32)
   if (lane >= mpw) return;  // no barriers in this kernel
   const int st = (blockDim.x >> 5) * mpw;  // slots per block
   const int slot = (threadIdx.x >> 5) * mpw + lane;
-  T *dd = reinterpret_cast<T *>(smem_raw) + slot;
-  T *ee = dd + (size_t)nmax * st;
+  using V = typename DEVec<T>::V;
+  const DEPair<T> de{reinterpret_cast<V *>(smem_raw) + slot, st};
   for (;;) {
     const int j = atomicAdd(next, 1);
     if (j >= njobs) return;
@@ -61,14 +61,11 @@ __global__ void __launch_bounds__(K2_MAX_WARPS * 32)
     }
     const T *din = G.d + (size_t)job.k * n;
     T *ein = G.e + (size_t)job.k * n;
-    for (int i = 0; i < n; i++) {
-      dd[(size_t)i * st] = din[i];
-      ee[(size_t)i * st] = ein[i];
-    }
+    for (int i = 0; i < n; i++) de.put(de.at(i), 0, din[i], ein[i]);
     Rec<T> *out = G.rec + (size_t)job.k * G.rcap;
     int ierr = 0;
-    const int nr = (method == QL_IMTQL2) ? ql_imtql2_fast(dd, ee, st, n, out, G.rcap, max_sweep, &ierr)
-                                         : ql_tql2_fast(dd, ee, st, n, out, G.rcap, max_sweep, &ierr);
+    const int nr = (method == QL_IMTQL2) ? ql_imtql2_fast_s<T>(de, n, out, G.rcap, max_sweep, &ierr)
+                                         : ql_tql2_fast_s<T>(de, n, out, G.rcap, max_sweep, &ierr);
     Meta mt;
     mt.nrec = nr < 0 ? 0 : nr;
     mt.pad = 0;
@@ -78,7 +75,7 @@ __global__ void __launch_bounds__(K2_MAX_WARPS * 32)
     } else {
       mt.overflow = 0;
       mt.ierr = ierr;
-      for (int i = 0; i < n; i++) ein[i] = dd[(size_t)i * st];  // unsorted eigenvalues over e, as k2_ql
+      for (int i = 0; i < n; i++) ein[i] = de.d(de.at(i), 0);  // unsorted eigenvalues over e, as k2_ql
     }
     G.meta[job.k] = mt;
   }

@@ -166,17 +166,20 @@ template <class T> int k1c_block(int n, size_t optin)
 }
 template <class T> size_t k2_smem_per_thread(int n) { return sizeof(T) * 2 * (size_t)n; }
 
-// Phase 2 matrices per warp: the largest power of two that still gives
-// each SM about three warps; two for batches of 1025 .. 2048 (measured on
-// B200: 8 per warp for 4096 matrices, 32 for 16384, 2 for 2048 at n = 32 ..
-// 256).  Smaller batches, such as the chunks of solve_host that run beside
-// another chunk's solve, keep the rule: one per warp would be faster alone
-// but crowds out the concurrent solve.
-inline int k2_mpw(long L, int sms)
+// Phase 2 matrices per warp: one while that is at most four warps an SM
+// (eight in FP32, whose rotations take fewer issue slots), else the smallest
+// power of two that is.  Each warp alone is bound by its chains' latency, up
+// to about one warp a scheduler; beyond, more lanes a warp cost less than
+// more warps.  Measured on B200 (phase 2, ms by matrices per warp): FP64 n=256
+// L=2048 1: 13.5, 2: 9.1, 4: 7.3, 8: 8.0; n=128 L=4096 4: 2.25, 8: 1.77, 16:
+// 1.91; n=45 L=6000 8: 0.46, 16: 0.37; n=512 L=256 1: 21.1, 2: 24.3; FP32
+// n=201 L=1000 1: 2.85, 2: 3.49; n=256 L=2048 2: 5.5, 4: 5.2, 8: 5.9.  (Taken
+// before the rotation loop was unrolled, which scales them alike.)
+template <class T> int k2_mpw(long L, int sms)
 {
-  const long target = (L > 1024 && L <= 2048) ? L / 2 : 3L * sms;
-  int m = 32;
-  while (m > 1 && (L + m - 1) / m < target) m >>= 1;
+  if (L <= (sizeof(T) == 8 ? 4L : 8L) * sms) return 1;
+  int m = 2;
+  while (m < 32 && (L + m - 1) / m > 4L * sms) m <<= 1;
   return m;
 }
 
@@ -694,7 +697,7 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
   }
   // phase 2: matrices per warp, then warps per block within the shared
   // memory budget (2n values per matrix)
-  p.k2mpw = k2_mpw(std::min(count, pl.Lc), dp.sms);
+  p.k2mpw = k2_mpw<T>(std::min(count, pl.Lc), dp.sms);
   if (opts && opts->ql_mpw > 0) {
     const int q = opts->ql_mpw;
     if (q > 32 || (q & (q - 1)) != 0) return cudaErrorInvalidValue;
@@ -703,10 +706,9 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
   int k2_mpb = 32;  // matrices per block, a multiple of k2mpw
   {
     const size_t per = k2_smem_per_thread<T>(n);
-    const size_t budget = std::min<size_t>((size_t)dp.smem_optin, 96 * 1024);
-    const int warps = (int)std::max<size_t>(
-        1, std::min<size_t>(std::max(1, std::min(K2_MAX_WARPS, 32 / p.k2mpw)), budget / (per * p.k2mpw)));
-    k2_mpb = warps * p.k2mpw;
+    // one warp per block: the device then spreads the warps evenly (n=128
+    // L=4096 FP64, 512 warps: 1.96 ms, in 171 blocks of three 2.56)
+    k2_mpb = p.k2mpw;
     if ((size_t)k2_mpb * per > (size_t)dp.smem_optin) {
       p.k2mpw = 1;
       k2_mpb = 1;
@@ -949,7 +951,7 @@ struct UnevenPlan {
   std::vector<UnevenItem> items;
   std::vector<UnevenWave> waves;
   std::vector<QJob> jobs;
-  int nstreams = 0, mpw = 4, method = QL_TQL2, max_sweep = 100;
+  int nstreams = 0, mpw = 0 /* automatic */, method = QL_TQL2, max_sweep = 100;
   size_t off_kid = 0, off_aoff = 0, off_woff = 0, off_groups = 0, off_jobs = 0, off_next = 0, off_region = 0;
   size_t region = 0, bytes = 0;
 };
@@ -1138,14 +1140,11 @@ cudaError_t launch_ql_queue(const UnevenPlan &up, const UnevenWave &wv, const QG
   cudaError_t err = dev_props(dp);
   if (err != cudaSuccess) return err;
   const size_t per = queue_slot_bytes<T>(wv.nmax);
-  const size_t budget = std::min<size_t>((size_t)dp.smem_optin, 96 * 1024);
-  int mpw = up.mpw;
-  int warps = (int)std::min<size_t>(std::max(1, std::min(K2_MAX_WARPS, 32 / mpw)), budget / (per * mpw));
-  if (warps < 1) {  // one slot per warp
-    mpw = 1;
-    warps = (int)std::min<size_t>(K2_MAX_WARPS, std::max<size_t>(1, budget / per));
-    if (per > (size_t)dp.smem_optin) return cudaErrorInvalidValue;
-  }
+  // one warp per block, as run() launches k2_ql
+  int mpw = up.mpw > 0 ? up.mpw : std::min(4, k2_mpw<T>(wv.njobs, dp.sms));
+  if (per * mpw > (size_t)dp.smem_optin) mpw = 1;
+  if (per > (size_t)dp.smem_optin) return cudaErrorInvalidValue;
+  const int warps = 1;
   const size_t smem = per * (size_t)mpw * warps;
   if ((err = set_smem(k2_ql_queue<T>, smem)) != cudaSuccess) return err;
   int nb = 0;
