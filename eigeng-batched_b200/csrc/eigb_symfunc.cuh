@@ -9,15 +9,16 @@
 //   SYMF_POW:  f(x) = pow(x, p) (p = 1/2 square root, -1 inverse, ...)
 //   SYMF_EXP:  f(x) = exp(p x)
 //
-// One CTA computes one 64 x 64 tile of Z for one matrix; only tiles on or
-// above the diagonal are computed and each off-diagonal tile is also
-// stored transposed (Z is symmetric).  The k loop stages 16-column panels
-// of V (rows of the tile) and of V scaled by f(w) (columns of the tile) in
-// shared memory, coalesced from the column-major V; each of the 256
-// threads accumulates a 4 x 4 register tile (rows and columns 16 apart,
-// so that a warp's shared-memory reads and its stores of Z are
-// contiguous).  FP64 on B200 runs SIMT FMAs at the rate of its FP64 tensor
-// path, so no tensor-core form is used.
+// The products run on the FP64 tensor cores (mma.sync m8n8k4) for both
+// types.  A warp computes one 32 x 32 tile of Z on or above the diagonal (the
+// 8 x 8 mma tiles below it are left out) and stores it to both triangles, so
+// Z is exactly symmetric.  With lane (g, q) = (lane / 4, lane % 4), the A
+// fragment V(i, k) and the B fragment V(j, k) of 8 rows and 4 columns are the
+// same picture, row g, column q, so one panel of V serves both; f(w_k) scales
+// B as it is loaded.
+//   n <= 32   one warp per matrix, fragments straight from global memory
+//   n <= 128  one CTA per matrix, a warp per tile: V is read once
+//   above     one CTA of 16 warps per 128 x 128 block of Z
 #pragma once
 #include "eigb_common.cuh"
 
@@ -25,9 +26,9 @@ namespace eigb {
 
 enum { SYMF_DIAG = 0, SYMF_POW = 1, SYMF_EXP = 2 };
 
-constexpr int SF_TILE = 64;  // tile of Z per CTA
-constexpr int SF_KC = 16;    // k panel
-constexpr int SF_LDP = SF_TILE + 4;
+constexpr int SF_KC = 16;     // columns of V per panel
+constexpr int SF_LD = 132;    // pitch of a panel: 4 mod 16 doubles, so that the fragment loads
+                              // (four columns, rows of 8) are free of bank conflicts
 
 template <class T> __device__ __forceinline__ T symf_apply(const int func, const T x, const T p)
 {
@@ -36,7 +37,7 @@ template <class T> __device__ __forceinline__ T symf_apply(const int func, const
   return x;
 }
 
-// upper-triangular tile index t -> (ti, tj), ti <= tj, row-major over the
+// upper-triangular tile index t -> (ti, tj), ti <= tj, row by row over the
 // upper triangle of an nt x nt tile grid
 __host__ __device__ __forceinline__ void symf_tile(int t, const int nt, int &ti, int &tj)
 {
@@ -47,75 +48,179 @@ __host__ __device__ __forceinline__ void symf_tile(int t, const int nt, int &ti,
   }
   tj = ti + t;
 }
-
-template <class T>
-__global__ void __launch_bounds__(256) k_symfunc(const long L, const int nm, const int n, const T *__restrict__ v,
-                                                 const T *__restrict__ w, T *__restrict__ z, const int func,
-                                                 const T p, const int ntiles)
+// the same, column by column
+__host__ __device__ __forceinline__ void sf_tile(int t, int &ti, int &tj)
 {
-  __shared__ __align__(16) T Vi[SF_KC][SF_LDP];  // V(tile rows, k)
-  __shared__ __align__(16) T Vj[SF_KC][SF_LDP];  // f(w_k) V(tile columns, k)
-  __shared__ T fw[SF_KC];
-  const long k = blockIdx.x / ntiles;
-  if (k >= L) return;
-  const int nt = (n + SF_TILE - 1) / SF_TILE;
-  int ti, tj;
-  symf_tile((int)(blockIdx.x % ntiles), nt, ti, tj);
-  const int i0 = ti * SF_TILE, j0 = tj * SF_TILE;
+  tj = 0;
+  while (t > tj) {
+    t -= tj + 1;
+    tj++;
+  }
+  ti = t;
+}
+
+__device__ __forceinline__ void sf_dmma(double (&d)[2], const double a, const double b)
+{
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+// the 32 x 32 tile at (i0, j0), i0 <= j0, to both triangles of Z
+template <class T>
+__device__ __forceinline__ void sf_store(T *Z, const int nm, const int n, const int i0, const int j0,
+                                         const double (&acc)[4][4][2])
+{
+  const int g = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+#pragma unroll
+  for (int x = 0; x < 4; x++)
+#pragma unroll
+    for (int y = 0; y < 4; y++) {
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int i = i0 + 8 * x + g, j = j0 + 8 * y + 2 * q + e;
+        if (i <= j && j < n) {
+          const T v = (T)acc[x][y][e];
+          Z[i + (size_t)j * nm] = v;
+          Z[j + (size_t)i * nm] = v;
+        }
+      }
+    }
+}
+
+// n <= 32, SFW_WARPS matrices per CTA
+constexpr int SFW_WARPS = 4;
+template <class T>
+__global__ void __launch_bounds__(32 * SFW_WARPS) k_symfunc_w(const long L, const int nm, const int n,
+                                                              const T *__restrict__ v, const T *__restrict__ w,
+                                                              T *__restrict__ z, const int func, const T p)
+{
+  const long k = (long)blockIdx.x * SFW_WARPS + (threadIdx.x >> 5);
+  if (k >= L) return;  // uniform per warp; no CTA barrier below
+  const int g = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
   const T *V = v + (size_t)k * nm * n;
   const T *W = w + (size_t)k * n;
-  T *Z = z + (size_t)k * nm * n;
-  const int t = threadIdx.x;
-  const int tr = t % 16, tc = t / 16;  // rows tr + 16x, columns tc + 16y of the tile (x, y < 4)
-  T acc[4][4];
+  double acc[4][4][2];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int x = 0; x < 4; x++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b] = T(0);
-
-  for (int kc = 0; kc < n; kc += SF_KC) {
-    if (t < SF_KC) fw[t] = (kc + t < n) ? symf_apply(func, W[kc + t], p) : T(0);
-    __syncthreads();  // fw ready; the previous panel is consumed
-    // panel loads: 16 columns x 64 rows each, 4 elements per thread per panel
+    for (int y = 0; y < 4; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
+  T a[8][4], f[8];  // all of V first: its loads overlap
 #pragma unroll
-    for (int q = 0; q < (SF_KC * SF_TILE) / 256; q++) {
-      const int e = t + 256 * q;
-      const int rr = e % SF_TILE, cc = e / SF_TILE;
-      const int kk = kc + cc;
-      const bool kin = kk < n;
-      const int ri = i0 + rr, rj = j0 + rr;
-      Vi[cc][rr] = (kin && ri < n) ? V[ri + (size_t)kk * nm] : T(0);
-      Vj[cc][rr] = (kin && rj < n) ? fw[cc] * V[rj + (size_t)kk * nm] : T(0);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < SF_KC; c++) {
-      T a[4], b[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        a[u] = Vi[c][tr + 16 * u];  // 16 consecutive rows per warp: one wavefront
-        b[u] = Vj[c][tc + 16 * u];
-      }
-#pragma unroll
-      for (int x = 0; x < 4; x++)
-#pragma unroll
-        for (int y = 0; y < 4; y++) acc[x][y] = fma(a[x], b[y], acc[x][y]);
-    }
-  }
-  // Z(i, j) = Z(j, i) = acc for i <= j (every element of an off-diagonal
-  // tile; the upper half of a diagonal tile), so Z is exactly symmetric
-#pragma unroll
-  for (int y = 0; y < 4; y++) {
-    const int j = j0 + tc + 16 * y;
+  for (int s = 0; s < 8; s++) {
+    const int c = 4 * s + q;
+    f[s] = c < n ? W[c] : T(0);
 #pragma unroll
     for (int x = 0; x < 4; x++) {
-      const int i = i0 + tr + 16 * x;
-      if (i < n && j < n && i <= j) {
-        Z[i + (size_t)j * nm] = acc[x][y];
-        if (i != j) Z[j + (size_t)i * nm] = acc[x][y];
+      const int i = 8 * x + g;
+      a[s][x] = (c < n && i < n) ? V[i + (size_t)c * nm] : T(0);
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < 8; s++) {
+    if (4 * s >= n) break;
+    const double fs = 4 * s + q < n ? (double)symf_apply(func, f[s], p) : 0.0;
+#pragma unroll
+    for (int y = 0; y < 4; y++) {
+      const double b = fs * (double)a[s][y];
+#pragma unroll
+      for (int x = 0; x <= y; x++) sf_dmma(acc[x][y], (double)a[s][x], b);
+    }
+  }
+  sf_store<T>(z + (size_t)k * nm * n, nm, n, 0, 0, acc);
+}
+
+// n > 32: block (bi, bj) of 128 x 128 of one matrix per CTA.  MAXT = 320: one
+// block (n <= 128), a warp per tile on or above the diagonal; 512: 16 warps,
+// one per tile of the block, those below the diagonal idle.  Two panels of
+// SF_KC columns in flight; off the diagonal a panel holds the rows of both.
+__host__ __device__ inline size_t symf_smem_bytes(int n)
+{
+  return sizeof(double) * 2 * (size_t)(n <= 128 ? 1 : 2) * SF_KC * SF_LD + sizeof(double) * (size_t)((n + 15) & ~15);
+}
+template <class T, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT == 320 ? 2 : 1) k_symfunc_tc(const int nm, const int n,
+                                                                         const T *__restrict__ v,
+                                                                         const T *__restrict__ w, T *__restrict__ z,
+                                                                         const int func, const T p, const int nblk)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool ONE = MAXT == 320;
+  const int per = ONE ? 1 : nblk * (nblk + 1) / 2;
+  const long k = blockIdx.x / per;
+  int bi = 0, bj = 0;
+  if (!ONE) sf_tile((int)(blockIdx.x % per), bi, bj);
+  const bool two = bi != bj;
+  const T *V = v + (size_t)k * nm * n;
+  const T *W = w + (size_t)k * n;
+  double *panel = reinterpret_cast<double *>(smem_raw);
+  constexpr int PS = (ONE ? 1 : 2) * SF_KC * SF_LD;
+  double *fw = panel + 2 * PS;
+  const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, warp = t >> 5, g = lane >> 2, q = lane & 3;
+  int ti, tj;
+  if (ONE) {
+    sf_tile(warp, ti, tj);
+  } else {
+    ti = warp & 3;
+    tj = warp >> 2;
+  }
+  const int i0 = 128 * bi + 32 * ti, j0 = 128 * bj + 32 * tj;
+  const bool act = i0 <= j0 && j0 < n;
+
+  for (int c = t; c < ((n + 15) & ~15); c += nt) fw[c] = c < n ? (double)symf_apply(func, W[c], p) : 0.0;
+  // panel of columns c0 .. c0+15: rows of the block rows bi (and bj)
+  auto fill = [&](const int c0, double *P) {
+    for (int h = 0; h < (two ? 2 : 1); h++) {
+      const int r0 = 128 * (h == 0 ? bi : bj);
+      const int rows = min(128, ((n - r0 + 31) & ~31));
+      for (int c = warp; c < SF_KC; c += nt >> 5) {
+        double *D = P + (h * SF_KC + c) * SF_LD;
+        const T *src = V + r0 + (size_t)(c0 + c) * nm;
+        for (int r = lane; r < rows; r += 32) {
+          if (c0 + c < n && r0 + r < n) {
+            if (sizeof(T) == 8) cp_async<8>(D + r, src + r);
+            else D[r] = (double)src[r];
+          } else {
+            D[r] = 0.0;
+          }
+        }
+      }
+    }
+    cp_async_commit();
+  };
+  double acc[4][4][2];
+#pragma unroll
+  for (int x = 0; x < 4; x++)
+#pragma unroll
+    for (int y = 0; y < 4; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
+  fill(0, panel);
+  int cur = 0;
+  for (int c0 = 0; c0 < n; c0 += SF_KC, cur ^= 1) {
+    cp_async_wait_all();
+    __syncthreads();
+    if (c0 + SF_KC < n) fill(c0 + SF_KC, panel + (cur ^ 1) * PS);
+    if (act) {
+      const double *PA = panel + cur * PS + q * SF_LD + 32 * ti + g;
+      const double *PB = panel + cur * PS + (two ? SF_KC * SF_LD : 0) + q * SF_LD + 32 * tj + g;
+      const bool diag = i0 == j0;
+#pragma unroll
+      for (int s = 0; s < SF_KC / 4; s++) {
+        double a[4], b[4];
+        const double f = fw[c0 + 4 * s + q];
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          a[x] = PA[4 * s * SF_LD + 8 * x];
+          b[x] = f * PB[4 * s * SF_LD + 8 * x];
+        }
+#pragma unroll
+        for (int y = 0; y < 4; y++)
+#pragma unroll
+          for (int x = 0; x < 4; x++)
+            if (x <= y || !diag) sf_dmma(acc[x][y], a[x], b[y]);
       }
     }
   }
+  if (act) sf_store<T>(z + (size_t)k * nm * n, nm, n, i0, j0, acc);
 }
 
 }  // namespace eigb

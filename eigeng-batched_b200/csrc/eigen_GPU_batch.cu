@@ -2279,11 +2279,22 @@ cudaError_t symfunc_run(long L, int nm, int n, const T *v, const T *w, T *z, int
     return cudaErrorInvalidValue;
   if (func < SYMF_DIAG || func > SYMF_EXP) return cudaErrorInvalidValue;
   if (v == z) return cudaErrorInvalidValue;  // Z is written while V is still read
-  const int nt = (n + SF_TILE - 1) / SF_TILE;
-  const int ntiles = nt * (nt + 1) / 2;
-  const long blocks = L * ntiles;
+  if (n <= 32) {
+    k_symfunc_w<T><<<(unsigned)((L + SFW_WARPS - 1) / SFW_WARPS), 32 * SFW_WARPS, 0, stream>>>(L, nm, n, v, w, z, func,
+                                                                                                (T)p);
+    return cudaGetLastError();
+  }
+  const int nblk = (n + 127) / 128, nb = (n + 31) / 32;
+  const long blocks = nblk == 1 ? L : L * nblk * (nblk + 1) / 2;
   if (blocks > 0x7fffffffL) return cudaErrorInvalidValue;
-  k_symfunc<T><<<(unsigned)blocks, 256, 0, stream>>>(L, nm, n, v, w, z, func, (T)p, ntiles);
+  const size_t smem = symf_smem_bytes(n);
+  cudaError_t err = cudaSuccess;
+  if (nblk == 1) {
+    k_symfunc_tc<T, 320><<<(unsigned)blocks, 32 * nb * (nb + 1) / 2, smem, stream>>>(nm, n, v, w, z, func, (T)p, nblk);
+  } else {
+    if ((err = set_smem(k_symfunc_tc<T, 512>, smem)) != cudaSuccess) return err;
+    k_symfunc_tc<T, 512><<<(unsigned)blocks, 512, smem, stream>>>(nm, n, v, w, z, func, (T)p, nblk);
+  }
   return cudaGetLastError();
 }
 
