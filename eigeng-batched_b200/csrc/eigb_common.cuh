@@ -254,23 +254,7 @@ __device__ __forceinline__ int warp_min_int(int x)
   return x;
 }
 
-// A team is the set of threads that cooperate on one matrix: one warp
-// (several independent matrices per CTA) or the whole CTA.
-struct WarpTeam {
-  int rank;  // 0..31
-  __device__ WarpTeam() : rank(threadIdx.x & 31) {}
-  __device__ __forceinline__ int size() const { return 32; }
-  __device__ __forceinline__ void sync() const { __syncwarp(); }
-  // Sum over the warp, result in every lane; the trailing __syncwarp orders
-  // the shared-memory accesses around it like the CTA barrier does.
-  template <class T> __device__ __forceinline__ T sum(T x, T *)
-  {
-    x = warp_sum(x);
-    __syncwarp();
-    return x;
-  }
-};
-
+// The threads that cooperate on one matrix: the whole CTA.
 struct CtaTeam {
   int rank;
   int nthr;

@@ -1,7 +1,8 @@
 // Batch kernels of the B200 eigensolver.
 //
 //   k_n1           n == 1 (eigen_GPU_batch.cu:36-54): w = a(1,1), a(1,1) = 1
-//   k1_warp        phase 1 for n <= 32: one warp per matrix, 4 per CTA
+//   k1_warp        phase 1 for n <= 32: one warp per matrix, 4 per CTA, the
+//                  matrix in registers (eigb_tridiag_warp.cuh)
 //   k1_cl          phase 1 for 32 < n <= 512 on a thread-block cluster, the
 //                  matrix in the cluster's distributed shared memory
 //   k1_reg<NB>     phase 1 for 32 < n <= 64: one CTA per matrix, the matrix
@@ -44,6 +45,7 @@
 #include "eigb_tridiag_cl.cuh"
 #include "eigb_tridiag_reg.cuh"
 #include "eigb_tridiag_sym.cuh"
+#include "eigb_tridiag_warp.cuh"
 #include "eigb_wave.cuh"
 
 namespace eigb {
@@ -102,12 +104,8 @@ __host__ __device__ __forceinline__ int packed_at(int r, int c) { return r + c *
 
 constexpr int K1W_NW = 4;       // warps (matrices) per CTA in k1_warp
 constexpr int K2_MAX_WARPS = 8; // warps per CTA in k2_ql at most
-constexpr int K1W_LD = 33;      // padded leading dimension, odd
 constexpr int K3W_NW = 4;       // warps per CTA in k3_warp
-constexpr int K3W_CH = 128;     // records staged per warp
-
-// per warp: S (K1W_LD x 32), beta[32], pv[32], red[72], ubuf[4*32], gram[3*32]
-template <class T> __host__ __device__ constexpr int k1w_slot() { return K1W_LD * 32 + 32 + 32 + 72 + 128 + 96; }
+constexpr int K3W_CH = 128;     // records staged per warp and buffer
 
 // threads per row in k1_cta (column ranges split across warps).  FP64
 // 128 < n <= 240 takes two, which with a smaller leading block in shared
@@ -139,32 +137,18 @@ __global__ void k_n1(const KP<T> p)
 }
 
 // ---------------------------------------------------------------- phase 1
+// Bound by instruction issue and the steps' exchanges, so by warps in
+// flight: registers bounded for four CTAs an SM (five, with spills, 0.71 ms).
+// B200, n=32 FP64 L=16384: 0.40 ms, the matrix in shared memory 0.66.
 template <class T>
-__global__ void __launch_bounds__(32 * K1W_NW) k1_warp(const KP<T> p)
+__global__ void __launch_bounds__(32 * K1W_NW, 4) k1_warp(const KP<T> p)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int wid = threadIdx.x >> 5;
   const long k = (long)blockIdx.x * K1W_NW + wid;
   if (k >= p.Lc) return;  // uniform per warp; no CTA barrier is used below
-  T *S = reinterpret_cast<T *>(smem_raw) + wid * k1w_slot<T>();
-  T *beta_s = S + K1W_LD * 32;
-  T *pv = beta_s + 32;
-  T *red = pv + 32;
-  T *ubuf = red + 72;
-  T *gram = ubuf + 128;
-  WarpTeam tm;
-  const int n = p.n, nm = p.nm, r = tm.rank;
-  T *A = mat_ptr(p, k);
-  const T *Ap = p.ap ? p.ap + (size_t)k * packed_size(n) : nullptr;
-  for (int c = 0; c < n; c++)
-    if (r <= c) S[r + c * K1W_LD] = Ap ? Ap[packed_at(r, c)] : A[r + (size_t)c * nm];
-  __syncwarp();
-  for (int c = 0; c < n; c++)
-    if (r > c && r < n) S[r + c * K1W_LD] = S[c + r * K1W_LD];
-  __syncwarp();
-  tridiag_qt<T, 1>(tm, S, K1W_LD, S, K1W_LD, n, n, p.d + k * n, p.e + k * n, beta_s, pv, pv, red, ubuf, gram);
-  if (r < n)
-    for (int c = 0; c < n; c++) A[r + (size_t)c * nm] = S[r + c * K1W_LD];
+  tridiag_warp<T>(mat_ptr(p, k), p.nm, p.n, p.ap ? p.ap + (size_t)k * packed_size(p.n) : nullptr, p.d + k * p.n,
+                  p.e + k * p.n, reinterpret_cast<T *>(smem_raw) + wid * tw_smem_elems());
 }
 
 // Shared-memory elements of k1_cta: red[72], beta[n], pv[n],
@@ -358,35 +342,43 @@ __global__ void __launch_bounds__(K2_MAX_WARPS * 32) k2_ql(const KP<T> p)
 }
 
 // ---------------------------------------------------------------- phase 3, n <= 32
-#define EIGB_ROT(I)                                   \
-  {                                                   \
-    const Rec<T> rr = *rp++;                          \
-    const T h0 = z[I], h1 = z[I + 1];                 \
-    z[I + 1] = fma(rr.c, h1, rr.s * h0);              \
-    z[I] = fma(-rr.s, h1, rr.c * h0);                 \
-    if (--mm == 0) break;                             \
-  }
-
-template <class T>
-__device__ __forceinline__ void apply_duff32(T (&z)[32], int cur, int mm, const Rec<T> *rp)
+// Rotations top, top-1, ..., top-cnt+1 (cnt >= 1, 0 <= top <= 30; records
+// rp[0..cnt)) on a row in registers.  Four columns at a time: a block wholly
+// inside the range loads its records together and runs without branches
+// (with a test per rotation each waited for its own record: k3_warp n=32
+// FP64 L=16384 0.60 -> 0.41 ms), the ends go rotation by rotation.
+template <class T> __device__ __forceinline__ void rot32(T &z0, T &z1, const Rec<T> r)
 {
-  // rotations cur, cur-1, ..., cur-mm+1 (mm >= 1, 0 <= cur <= 30)
-  switch (cur) {
-    case 30: EIGB_ROT(30) case 29: EIGB_ROT(29) case 28: EIGB_ROT(28) case 27: EIGB_ROT(27)
-    case 26: EIGB_ROT(26) case 25: EIGB_ROT(25) case 24: EIGB_ROT(24) case 23: EIGB_ROT(23)
-    case 22: EIGB_ROT(22) case 21: EIGB_ROT(21) case 20: EIGB_ROT(20) case 19: EIGB_ROT(19)
-    case 18: EIGB_ROT(18) case 17: EIGB_ROT(17) case 16: EIGB_ROT(16) case 15: EIGB_ROT(15)
-    case 14: EIGB_ROT(14) case 13: EIGB_ROT(13) case 12: EIGB_ROT(12) case 11: EIGB_ROT(11)
-    case 10: EIGB_ROT(10) case 9: EIGB_ROT(9) case 8: EIGB_ROT(8) case 7: EIGB_ROT(7)
-    case 6: EIGB_ROT(6) case 5: EIGB_ROT(5) case 4: EIGB_ROT(4) case 3: EIGB_ROT(3)
-    case 2: EIGB_ROT(2) case 1: EIGB_ROT(1) case 0: EIGB_ROT(0)
-    default: break;
+  const T h0 = z0, h1 = z1;
+  z1 = fma(r.c, h1, r.s * h0);
+  z0 = fma(-r.s, h1, r.c * h0);
+}
+template <class T>
+__device__ __forceinline__ void apply_blocks32(T (&z)[32], const int top, const int cnt, const Rec<T> *rp)
+{
+  const int bot = top - cnt + 1;
+#pragma unroll
+  for (int b = 7; b >= 0; b--) {
+    const int hi = b == 7 ? 30 : 4 * b + 3, lo = 4 * b;
+    if (top < lo) continue;
+    if (bot > hi) break;
+    const Rec<T> *q = rp + (top - hi);
+    if (top >= hi && bot <= lo) {
+      Rec<T> r[4];
+#pragma unroll
+      for (int u = 0; u <= hi - lo; u++) r[u] = q[u];
+#pragma unroll
+      for (int u = 0; u <= hi - lo; u++) rot32(z[hi - u], z[hi - u + 1], r[u]);
+    } else {
+#pragma unroll
+      for (int u = 0; u <= hi - lo; u++)
+        if (hi - u <= top && hi - u >= bot) rot32(z[hi - u], z[hi - u + 1], q[u]);
+    }
   }
 }
-#undef EIGB_ROT
 
 template <class T> struct K3WSlot {
-  Rec<T> rbuf[K3W_CH];
+  Rec<T> rbuf[2 * K3W_CH];
   T sd[32], se[32], sdd[32];
   int inv[32], pos[32];
   int ierr, nrec, done;
@@ -440,12 +432,18 @@ __global__ void __launch_bounds__(32 * K3W_NW) k3_warp(const KP<T> p)
   K3WSlot<T> &sl = reinterpret_cast<K3WSlot<T> *>(smem_raw)[wid];
   const int n = p.n, nm = p.nm, r = threadIdx.x & 31;
   const T *A = mat_ptr(p, k);
-  // Z = Q: phase 1 left M = Q^T in a, so Z(r, c) = M(c, r) = a[c + r*nm]
-  T z[32];
-#pragma unroll
-  for (int c = 0; c < 32; c++) z[c] = (r < n && c < n) ? A[c + (size_t)r * nm] : T(0);
-
   const Meta mt = p.meta[k];
+  const Rec<T> *src = p.rec + (size_t)k * p.rcap;
+  auto stage = [&](const int base, Rec<T> *dst) {
+    const int cnt = min(K3W_CH, mt.nrec - base);
+    for (int q = r; q < cnt; q += 32) cp_async<sizeof(Rec<T>)>(dst + q, src + base + q);
+    cp_async_commit();
+  };
+  if (!mt.overflow) stage(0, sl.rbuf);
+  T z[32];  // Z = Q
+#pragma unroll
+  for (int c = 0; c < 32; c++) z[c] = (r < n && c < n) ? A[r + (size_t)c * nm] : T(0);
+
   int cur = 0, rem = 0;
   // applies one staged chunk of records (segments may continue across chunks)
   auto apply = [&](const Rec<T> *b, int nr) {
@@ -458,7 +456,7 @@ __global__ void __launch_bounds__(32 * K3W_NW) k3_warp(const KP<T> p)
         continue;
       }
       const int mm = min(rem, nr - q);
-      apply_duff32(z, cur, mm, b + q);
+      apply_blocks32(z, cur, mm, b + q);
       q += mm;
       rem -= mm;
       cur -= mm;
@@ -467,14 +465,14 @@ __global__ void __launch_bounds__(32 * K3W_NW) k3_warp(const KP<T> p)
   T dr;
   int ierr;
   if (!mt.overflow) {
-    const Rec<T> *src = p.rec + (size_t)k * p.rcap;
-    for (int base = 0; base < mt.nrec; base += K3W_CH) {
-      const int cnt = min(K3W_CH, mt.nrec - base);
-      for (int q = r; q < cnt; q += 32) sl.rbuf[q] = src[base + q];
+    // two buffers: the next chunk is copied in while this one is applied
+    for (int base = 0, cb = 0; base < mt.nrec; base += K3W_CH, cb ^= 1) {
+      cp_async_wait_all();
       __syncwarp();
-      apply(sl.rbuf, cnt);
-      __syncwarp();
+      if (base + K3W_CH < mt.nrec) stage(base + K3W_CH, sl.rbuf + (cb ^ 1) * K3W_CH);
+      apply(sl.rbuf + cb * K3W_CH, min(K3W_CH, mt.nrec - base));
     }
+    cp_async_wait_all();
     dr = (r < n) ? p.e[k * n + r] : T(0);
     ierr = mt.ierr;
   } else {

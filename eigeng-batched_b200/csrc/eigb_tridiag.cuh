@@ -13,7 +13,7 @@
 // (4/3 n^3 flops); the QL rotations are later applied to Q directly, which
 // gives the same eigenvectors Q * Z_T up to rounding.
 //
-// Thread mapping: the team (one warp, or the whole CTA) owns the rows of
+// Thread mapping: the team (the CTA) owns the rows of
 // the full symmetric n x n matrix S (column-major, leading dimension ld).
 // The team's nt threads form SPLIT groups of nr = nt/SPLIT threads; thread
 // t owns row r = t % nr and, within every row operation, the h-th of SPLIT

@@ -607,7 +607,7 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
   p.rcap = pl.rcap;
 
   // launch geometry
-  const size_t k1w_smem = sizeof(T) * k1w_slot<T>() * K1W_NW;
+  const size_t k1w_smem = sizeof(T) * tw_smem_elems() * K1W_NW;
   const size_t k3w_smem = sizeof(K3WSlot<T>) * K3W_NW;
   // phase 3: one row per thread up to 512 rows, two above
   bool ztm = pl.ztm != 0 && n > 32;
@@ -856,7 +856,7 @@ cudaError_t launch_params(long L, int n, int *grp, int *tb, int *gr, int *th, in
     *gr = K1W_NW;
     *th = 32 * K1W_NW;
     *tb = (int)((lc + K1W_NW - 1) / K1W_NW);
-    *sh = (int)(sizeof(T) * k1w_slot<T>() * K1W_NW);
+    *sh = (int)(sizeof(T) * tw_smem_elems() * K1W_NW);
   } else if (n <= 128) {  // the register form: NB x NB warps
     const int nb = (n + 31) / 32;
     *grp = *th = 32 * nb * nb;
