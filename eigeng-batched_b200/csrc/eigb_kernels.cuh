@@ -256,15 +256,17 @@ __global__ void __launch_bounds__(32 * SPLIT, 1024 / (32 * SPLIT)) k1_cl(const K
 }
 
 // Reduction of k1_sym<T, NW, RS, CN>: NW warps, RS blocks of a warp in
-// registers, CN CTAs per matrix (see eigb_tridiag_sym.cuh and sym_cfg).
+// registers, CN CTAs per matrix (see eigb_tridiag_sym.cuh and sym_cfg), of the
+// leading m x m block down to order `stop`.
 template <class T, int NW, int RS, int CN, int MB>
-__global__ void __launch_bounds__(32 * NW, MB) k1_sym(const KP<T> p)
+__global__ void __launch_bounds__(32 * NW, MB) k1_sym(const KP<T> p, const int m, const int stop)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const long k = blockIdx.x / CN;
   unsigned char *v = p.vw + (size_t)k * p.vstride;
-  tridiag_sym<T, NW, RS, CN>(mat_ptr(p, k), p.nm, p.n, p.ap ? p.ap + (size_t)k * packed_size(p.n) : nullptr,
-                             p.d + k * p.n, p.e + k * p.n, reinterpret_cast<T *>(v + fq_off_v(p.n)), fq_ldv(p.n),
+  tridiag_sym<T, NW, RS, CN>(mat_ptr(p, k), p.nm, m, stop, m == p.n,
+                             p.ap && m == p.n ? p.ap + (size_t)k * packed_size(p.n) : nullptr, p.d + k * p.n,
+                             p.e + k * p.n, reinterpret_cast<T *>(v + fq_off_v(p.n)), fq_ldv(p.n),
                              reinterpret_cast<double *>(v), reinterpret_cast<T *>(smem_raw));
 }
 

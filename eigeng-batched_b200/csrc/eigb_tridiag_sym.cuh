@@ -170,9 +170,13 @@ __device__ __forceinline__ void sym_block(const int lane, const T *__restrict__ 
 //            gets all of them (or their totals, sym_homes) and computes the
 //            tail for all rows itself
 //   barrier  (cluster)
+//
+// Reduces the leading n x n block of A down to order `stop` (0: to the end),
+// where it leaves the updated leading block in A's upper triangle for a call
+// with fewer warps or CTAs; `first` is the call on the whole matrix.
 template <class T, int NW, int RS, int CN>
-__device__ void tridiag_sym(T *A, const int nm, const int n, const T *Ap, T *d_out, T *e_out, T *V, const int ldv,
-                            double *beta_out, T *sm)
+__device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, const bool first, const T *Ap, T *d_out,
+                            T *e_out, T *V, const int ldv, double *beta_out, T *sm)
 {
   constexpr int NT = 32 * NW;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -236,6 +240,7 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const T *Ap, T *d_o
     x[0] = x[32] = x[64] = T(0);
     cb[((n - 1) & 1) * nr + r] = elem(r, n - 1);
   }
+  if (first && rank == 0 && t == 0) e_out[n - 1] = T(0);
   if (t < 8) sc[t] = T(0);
   if (t < 64) dotp[t] = T(0);  // and sg
   if (CN > 1) cg::this_cluster().sync();
@@ -310,7 +315,7 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const T *Ap, T *d_o
         w = fma(alpha, u, beta * fma(-anorm, c, y));
         const T x = fma(w, ul, fma(u, wi, c));
         if (r == i) {
-          if (rank == 0) d_out[i] = x;
+          if (rank == 0 && i >= stop) d_out[i] = x;
         } else {
           v = x;
         }
@@ -322,6 +327,31 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const T *Ap, T *d_o
       sig = fma(v, v, sig);
     }
     if (i == 0) break;
+    if (i < stop) {  // i = stop - 1: the pending update alone, and the block goes out
+      __syncthreads();
+      auto out = [&](const int l, auto get) {
+        const int g = l * CN + rank;
+        int C = 0;
+        while ((C + 1) * (C + 2) / 2 <= g) C++;
+        const int R = g - C * (C + 1) / 2;
+        const T *xR = uwv + 96 * R, *xC = uwv + 96 * C;
+#pragma unroll
+        for (int x = 0; x < 32; x++) {
+          const int r = 2 * lr + 8 * ((x >> 3) ^ xj) + ((x >> 2) & 1), c = 2 * lc + 16 * (((x >> 1) & 1) ^ xh) + (x & 1);
+          const T v = fma(xR[32 + r], xC[c], fma(xR[r], xC[32 + c], get(x)));
+          if (32 * R + r <= 32 * C + c) A[32 * R + r + (size_t)(32 * C + c) * nm] = v;
+        }
+      };
+      const int nout = (stop / 32) * (stop / 32 + 1) / 2;
+      for (int l = RS * NW + warp; l * CN + rank < nout; l += NW) {
+        const T *B = blk + (size_t)(l - RS * NW) * 1024 + 2 * lane;
+        out(l, [&](const int x) { return B[(x >> 1) * 64 + (x & 1)]; });
+      }
+#pragma unroll
+      for (int s = 0; s < RS; s++)
+        if ((s * NW + warp) * CN + rank < nout) out(s * NW + warp, [&](const int x) { return S[s][x]; });
+      return;
+    }
     sig = warp_sum(sig);
     if (lane == 0) sg[warp] = sig;
     __syncthreads();
@@ -452,10 +482,7 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const T *Ap, T *d_o
       cg::this_cluster().sync();
     }
   }
-  if (t == 0 && rank == 0) {
-    e_out[n - 1] = T(0);
-    beta_out[0] = 0.0;
-  }
+  if (t == 0 && rank == 0) beta_out[0] = 0.0;
 }
 
 }  // namespace eigb

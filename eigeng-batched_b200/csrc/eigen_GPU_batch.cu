@@ -359,7 +359,7 @@ template <class T> SymCfg sym_cfg(int n)
   if (n <= 736) return {8, 4, 4, 1};
   return {8, 4, 8, 1};
 }
-template <class T> using SymKernel = void (*)(const KP<T>);
+template <class T> using SymKernel = void (*)(const KP<T>, const int, const int);
 template <class T> SymKernel<T> sym_kernel(const SymCfg &c)
 {
   if constexpr (sizeof(T) == 8) {
@@ -385,6 +385,23 @@ template <class T> SymKernel<T> sym_kernel(const SymCfg &c)
 template <class T> size_t sym_smem(int n, const SymCfg &c)
 {
   return sizeof(T) * sym_smem_elems(n, c.nw, c.rs, c.cn);
+}
+// Order at which a reduction that began at n hands the leading block over to a
+// launch with fewer CTAs or warps (0: none).  A matrix keeps its SMs to the
+// last step otherwise, and the last steps have little to do; where the batch
+// takes more than one wave of CTAs, another launch packs the small blocks
+// closer.  Measured on B200 (the reduction, ms, without / with): FP64 n=160
+// L=3000 4.20 / 3.84, n=256 L=2048 9.68 / 8.39, n=512 L=256 14.0 / 10.3, n=1000
+// L=32 26.9 / 18.2; FP32 n=201 L=1000 1.57 / 1.37, n=512 L=256 6.80 / 5.30,
+// n=1000 L=32 14.1 / 9.3.  In a single wave it costs: FP64 n=512 L=32 1.76 /
+// 2.12.
+template <class T> int sym_next(int n, long cnt, const SymCfg &c, int sms)
+{
+  if (cnt * c.cn <= (long)sms * c.mb) return 0;
+  const int at64[] = {736, 512, 352, 256, 128, 0}, at32[] = {736, 512, 384, 160, 0};
+  const int *at = sizeof(T) == 8 ? at64 : at32;
+  while (*at >= n) at++;
+  return *at;
 }
 template <class T> cudaLaunchConfig_t sym_launch(int n, const SymCfg &c, long cnt, cudaStream_t st,
                                                  cudaLaunchAttribute *at)
@@ -425,7 +442,11 @@ template <class T> bool sym_usable(int n, const SymCfg &c, const DevProps &dp)
   return clusters >= 1;
 }
 
-// formation of Q: column tiles per warp and warps per 8 rows by order
+// formation of Q: column tiles per warp and warps per 8 rows by order.  Two
+// CTAs an SM (128 registers) beat one of longer tiles up to 256, not above
+// (B200, ms, 32 tiles and one CTA / 16 and two): FP64 n=200 L=2048 2.01 /
+// 1.53, n=256 3.18 / 2.50, n=512 L=256 3.29 / 3.94, n=1000 L=32 3.41 / 4.86;
+// FP32 n=201 L=1000 1.29 / 0.97.
 template <class T> struct FormQ {
   void (*kern)(const KP<T>, const int);
   int rows, nbuf;
@@ -435,20 +456,27 @@ template <class T> FormQ<T> form_q_cfg(int n, size_t optin)
 {
   FormQ<T> f;
   if (n <= 128) f.kern = k1_formq<T, 16, 1, 2>;
-  else if (n <= 256) f.kern = k1_formq<T, 32, 1, 1>;
+  else if (n <= 256) f.kern = k1_formq<T, 16, 2, 2>;
   else if (n <= 512) f.kern = k1_formq<T, 32, 2, 1>;
   else f.kern = k1_formq<T, 32, 4, 1>;
-  f.rows = fq_rows(n <= 256 ? 1 : (n <= 512 ? 2 : 4));
+  f.rows = fq_rows(n <= 128 ? 1 : (n <= 512 ? 2 : 4));
   f.nbuf = fq_smem_bytes(n, 2) <= optin ? 2 : 1;
   f.smem = fq_smem_bytes(n, f.nbuf);
   return f;
 }
-template <class T> cudaError_t launch_sym(const KP<T> &p, const SymCfg &c, const FormQ<T> &f, long cnt, cudaStream_t st)
+template <class T>
+cudaError_t launch_sym(const KP<T> &p, const DevProps &dp, const FormQ<T> &f, long cnt, cudaStream_t st)
 {
-  cudaLaunchAttribute at[1];
-  cudaLaunchConfig_t cfg = sym_launch<T>(p.n, c, cnt, st, at);
-  const cudaError_t err = cudaLaunchKernelEx(&cfg, sym_kernel<T>(c), p);
-  if (err != cudaSuccess) return err;
+  for (int m = p.n; m > 0;) {
+    const SymCfg c = sym_cfg<T>(m);
+    int stop = sym_next<T>(m, cnt, c, dp.sms);
+    if (stop && !sym_usable<T>(stop, sym_cfg<T>(stop), dp)) stop = 0;  // also sets the next kernel's attributes
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = sym_launch<T>(m, c, cnt, st, at);
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, sym_kernel<T>(c), p, m, stop);
+    if (err != cudaSuccess) return err;
+    m = stop;
+  }
   const long warps = cnt * fq_blocks(p.n);
   k1_factor<T><<<(unsigned)((warps + K1F_NW - 1) / K1F_NW), 32 * K1F_NW, 0, st>>>(p);
   f.kern<<<(unsigned)(cnt * ((p.n + f.rows - 1) / f.rows)), 256, f.smem, st>>>(p, f.nbuf);
@@ -750,7 +778,7 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
     } else if (k1_in_regs) {
       k1_reg<T, 2><<<(unsigned)cnt, 32 * 4, k1c_smem, st>>>(q);
     } else if (k1_symm) {
-      const cudaError_t e = launch_sym<T>(q, k1_symc, k1_fq, cnt, st);
+      const cudaError_t e = launch_sym<T>(q, dp, k1_fq, cnt, st);
       if (e != cudaSuccess && lerr == cudaSuccess) lerr = e;
     } else {
       launch_k1<T>(q, (unsigned)cnt, k1c_nt, k1c_smem, st);
