@@ -5,12 +5,12 @@
 //                  matrix in registers (eigb_tridiag_warp.cuh)
 //   k1_cl          phase 1 for 32 < n <= 512 on a thread-block cluster, the
 //                  matrix in the cluster's distributed shared memory
-//   k1_reg<NB>     phase 1 for 32 < n <= 64: one CTA per matrix, the matrix
-//                  in registers (eigb_tridiag_reg.cuh)
-//   k1_sym<...>    phase 1 for n > 64, the reduction: the upper triangle in
+//   k1_reg<NB>     FP32 phase 1 for 32 < n <= 64: one CTA per matrix, the
+//                  matrix in registers (eigb_tridiag_reg.cuh)
+//   k1_sym<...>    phase 1 for larger n (FP64: n > 32), the reduction: the upper triangle in
 //                  registers and shared memory of one CTA or of a cluster
 //                  (eigb_tridiag_sym.cuh)
-//   k1_factor, k1_formq  phase 1 for n > 64, Q from the reflectors on the
+//   k1_factor, k1_formq  phase 1 after k1_sym, Q from the reflectors on the
 //                  FP64 tensor cores (eigb_formq.cuh)
 //   k1_cta<SPLIT>  phase 1 where the device cannot run k1_sym's cluster: one
 //                  CTA per matrix; the leading block that fits is staged in

@@ -242,7 +242,7 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
   }
   if (first && rank == 0 && t == 0) e_out[n - 1] = T(0);
   if (t < 8) sc[t] = T(0);
-  if (t < 64) dotp[t] = T(0);  // and sg
+  for (int q = t; q < 64; q += NT) dotp[q] = T(0);  // and sg
   if (CN > 1) cg::this_cluster().sync();
   else __syncthreads();
 

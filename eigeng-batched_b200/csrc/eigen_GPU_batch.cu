@@ -193,7 +193,7 @@ template <class T> struct Plan {
   int zsplit = 1;     // phase 3: CTAs per matrix
   int ztm = 0;        // phase 3: rows of Z in tensor memory instead of shared memory
   size_t off_d = 0, off_e = 0, off_meta = 0, off_rec = 0, off_z = 0, bytes = 0;
-  // reflectors of phase 1 (n > 64): in the place of the records, which phase
+  // reflectors of phase 1 (n > 32): in the place of the records, which phase
   // 2 writes later, unless a caller's rec_cap leaves that too small
   size_t off_v = 0, vstride = 0;
 };
@@ -266,8 +266,8 @@ cudaError_t make_plan(long L, int nm, int n, const DevProps &dp, Plan<T> &pl, co
   }
   const bool zglob = n > 32 && pl.zrows == 0;
   const size_t rec_b = sizeof(Rec<T>) * (size_t)pl.rcap;
-  const bool vown = n > 64 && (rec_b < fq_bytes<T>(n) || rec_b % 16 != 0);
-  pl.vstride = n > 64 ? (vown ? fq_bytes<T>(n) : rec_b) : 0;
+  const bool vown = n > 32 && (rec_b < fq_bytes<T>(n) || rec_b % 16 != 0);
+  pl.vstride = n > 32 ? (vown ? fq_bytes<T>(n) : rec_b) : 0;
   const size_t per = sizeof(T) * 2 * (size_t)n + sizeof(Meta) + rec_b + (vown ? pl.vstride : 0) +
                      (zglob ? sizeof(T) * (size_t)n * n : 0);
   long lc = (long)(kWsBudget / per);
@@ -319,11 +319,12 @@ template <class K> cudaError_t set_smem(K kern, size_t bytes)
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// phase 1 in registers for 32 < n <= 64 (2 x 2 blocks of 32 x 32).  Above,
-// k1_sym with its separate formation of Q is faster (B200, phase 1 in ms,
-// this form / k1_sym): FP64 n=64 L=20000 4.43 / 5.12, n=96 L=8000 7.68 /
-// 4.35, n=128 L=4096 6.88 / 4.28; FP32 n=64 2.02 / 3.47, n=128 3.34 / 2.65.
-inline bool reg_form(int n) { return n > 32 && n <= 64; }
+// FP32 phase 1 in registers for 32 < n <= 64 (2 x 2 blocks of 32 x 32).  In
+// FP64, and above, k1_sym with its separate formation of Q is faster (B200,
+// phase 1 in ms, this form / k1_sym): FP64 n=45 L=6000 0.80 / 0.75, n=64
+// L=20000 4.43 / 3.61, n=96 L=8000 7.68 / 3.98, n=128 L=4096 6.88 / 3.85; FP32
+// n=64 2.02 / 2.83, n=128 3.34 / 2.58.
+template <class T> bool reg_form(int n) { return sizeof(T) == 4 && n > 32 && n <= 64; }
 template <class T> size_t k1r_smem_bytes(int n) { return sizeof(T) * reg_smem_elems<2>(n); }
 
 // k1_sym: warps, blocks per warp in registers and CTAs per matrix
@@ -332,17 +333,21 @@ struct SymCfg {
 };
 // Measured on B200 (the reduction alone, ms).  Where several matrices fit an
 // SM, small CTAs with few blocks in registers win, their step chains hiding
-// one another: FP64 n=128 L=4096 4 warps x 1 block, three CTAs 3.04, x 2
+// one another: FP64 n=64 L=20000 one warp x 2 blocks 2.85, two x 1 3.26, four
+// x 1 4.43; n=96 L=8000 two x 1, six CTAs 3.07, four x 1 3.40; n=128 L=4096 4 warps x 1 block, three CTAs 3.04, x 2
 // blocks, two CTAs 3.48, 8 x 2, one CTA 5.62; n=160 L=3000 4.65 / 4.05 /
 // 5.69.  From n = 161 on 4 warps no longer have two CTAs an SM (n=192 L=2048
 // 6.58 against 5.20 with 8).  Above 256 the fewest CTAs that hold the
 // triangle: n=512 L=256 4 CTAs 13.4, 8 CTAs 28.8; n=384 L=512 15.3 / 36.8;
-// n=736 L=64 8 CTAs 15.6, 16 CTAs 29.2.  FP32: n=160 L=3000 4 x 1 2.14, 8 x 1
+// n=736 L=64 8 CTAs 15.6, 16 CTAs 29.2.  FP32: n=96 L=8000 2 x 1,
+// eight CTAs 1.67, 4 x 1 2.07; n=128 L=4096 2 x 2 1.66, 4 x 1 1.76; n=160 L=3000 4 x 1 2.14, 8 x 1
 // 2.80; n=224 L=2048 4.33 / 3.53; n=256 8 x 1 7.06, 4 x 4 5.04, 8 x 4 6.28;
 // n=288 L=1024 4 x 4 5.79, 8 x 4 4.03; n=1000 L=32 8 CTAs 14.2, 16 21.1.
 template <class T> SymCfg sym_cfg(int n)
 {
   if (sizeof(T) == 8) {
+    if (n <= 64) return {1, 2, 1, 8};
+    if (n <= 96) return {2, 1, 1, 6};
     if (n <= 128) return {4, 1, 1, 3};
     if (n <= 160) return {4, 2, 1, 2};
     if (n <= 256) return {8, 2, 1, 1};
@@ -351,6 +356,8 @@ template <class T> SymCfg sym_cfg(int n)
     if (n <= 736) return {8, 2, 8, 1};
     return {8, 2, 16, 1};
   }
+  if (n <= 96) return {2, 1, 1, 8};
+  if (n <= 128) return {2, 2, 1, 6};
   if (n <= 160) return {4, 1, 1, 4};
   if (n <= 224) return {8, 1, 1, 2};
   if (n <= 256) return {4, 4, 1, 2};
@@ -363,6 +370,8 @@ template <class T> using SymKernel = void (*)(const KP<T>, const int, const int)
 template <class T> SymKernel<T> sym_kernel(const SymCfg &c)
 {
   if constexpr (sizeof(T) == 8) {
+    if (c.nw == 1) return k1_sym<T, 1, 2, 1, 8>;
+    if (c.nw == 2) return k1_sym<T, 2, 1, 1, 6>;
     if (c.nw == 4) return c.rs == 1 ? k1_sym<T, 4, 1, 1, 3> : k1_sym<T, 4, 2, 1, 2>;
     switch (c.cn) {
       case 1: return k1_sym<T, 8, 2, 1, 1>;
@@ -372,6 +381,7 @@ template <class T> SymKernel<T> sym_kernel(const SymCfg &c)
       default: return k1_sym<T, 8, 2, 16, 1>;
     }
   } else {
+    if (c.nw == 2) return c.rs == 1 ? k1_sym<T, 2, 1, 1, 8> : k1_sym<T, 2, 2, 1, 6>;
     if (c.nw == 4) return c.rs == 1 ? k1_sym<T, 4, 1, 1, 4> : k1_sym<T, 4, 4, 1, 2>;
     if (c.rs == 1) return k1_sym<T, 8, 1, 1, 2>;
     switch (c.cn) {
@@ -424,7 +434,7 @@ template <class T> cudaLaunchConfig_t sym_launch(int n, const SymCfg &c, long cn
 template <class T> bool sym_usable(int n, const SymCfg &c, const DevProps &dp)
 {
   const size_t smem = sym_smem<T>(n, c);
-  if (n <= 64 || smem > (size_t)dp.smem_optin) return false;
+  if (n <= 32 || reg_form<T>(n) || smem > (size_t)dp.smem_optin) return false;
   SymKernel<T> kern = sym_kernel<T>(c);
   if (set_smem(kern, smem) != cudaSuccess) return false;
   if (c.cn == 1) return true;
@@ -455,7 +465,8 @@ template <class T> struct FormQ {
 template <class T> FormQ<T> form_q_cfg(int n, size_t optin)
 {
   FormQ<T> f;
-  if (n <= 128) f.kern = k1_formq<T, 16, 1, 2>;
+  if (n <= 64) f.kern = k1_formq<T, 8, 1, 3>;
+  else if (n <= 128) f.kern = k1_formq<T, 16, 1, 2>;
   else if (n <= 256) f.kern = k1_formq<T, 16, 2, 2>;
   else if (n <= 512) f.kern = k1_formq<T, 32, 2, 1>;
   else f.kern = k1_formq<T, 32, 4, 1>;
@@ -647,7 +658,7 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
   const int k1c_nt = k1c_threads<T>(n);
   const int red_form = tuned_reduce((int)sizeof(T), n);
   const bool k1_cluster = red_form == EIGEN_GPU_REDUCE_CLUSTER && k1cl_usable<T>(n, dp);
-  const bool k1_in_regs = !k1_cluster && reg_form(n);
+  const bool k1_in_regs = !k1_cluster && reg_form<T>(n);
   const SymCfg k1_symc = sym_cfg<T>(n);
   const bool k1_symm = !k1_cluster && sym_usable<T>(n, k1_symc, dp);
   const FormQ<T> k1_fq = form_q_cfg<T>(n, (size_t)dp.smem_optin);
@@ -751,7 +762,8 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
     if (k1_cluster) {
       // attributes set by k1cl_usable
     } else if (k1_in_regs) {
-      if ((err = set_smem(k1_reg<T, 2>, k1c_smem)) != cudaSuccess) return err;
+      if constexpr (sizeof(T) == 4)
+        if ((err = set_smem(k1_reg<T, 2>, k1c_smem)) != cudaSuccess) return err;
     } else if (k1_symm) {  // k1_sym's attributes set by sym_usable
       if ((err = set_smem(k1_fq.kern, k1_fq.smem)) != cudaSuccess) return err;
     } else if ((err = set_k1_smem<T>(n, k1c_smem)) != cudaSuccess) {
@@ -776,7 +788,7 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
       const cudaError_t e = launch_k1cl<T>(q, cnt, st);
       if (e != cudaSuccess && lerr == cudaSuccess) lerr = e;
     } else if (k1_in_regs) {
-      k1_reg<T, 2><<<(unsigned)cnt, 32 * 4, k1c_smem, st>>>(q);
+      if constexpr (sizeof(T) == 4) k1_reg<T, 2><<<(unsigned)cnt, 32 * 4, k1c_smem, st>>>(q);
     } else if (k1_symm) {
       const cudaError_t e = launch_sym<T>(q, dp, k1_fq, cnt, st);
       if (e != cudaSuccess && lerr == cudaSuccess) lerr = e;

@@ -1,4 +1,4 @@
-"""Phase 1 for n > 64: the reduction on the upper triangle in registers and
+"""Phase 1 for n > 32: the reduction on the upper triangle in registers and
 shared memory (k1_sym) and the formation of Q from its reflectors
 (k1_factor, k1_formq), at the edges of their 32 x 32 blocks, of the 16
 reflectors of a block factor and of the orders from which a matrix takes
@@ -17,7 +17,7 @@ torch = pytest.importorskip("torch")
 
 pytestmark = pytest.mark.gpu
 
-F64 = [65, 66, 80, 81, 96, 97, 127, 128, 129, 160, 161, 191, 256, 257, 288, 352, 353, 512, 513, 736, 737, 1024]
+F64 = [33, 34, 47, 48, 49, 63, 64, 65, 66, 80, 81, 96, 97, 127, 128, 129, 160, 161, 191, 256, 257, 288, 352, 353, 512, 513, 736, 737, 1024]
 F32 = [65, 97, 128, 129, 160, 161, 193, 224, 225, 256, 257, 384, 385, 512, 513, 736, 737, 1024]
 
 
