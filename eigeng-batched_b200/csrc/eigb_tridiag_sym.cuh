@@ -155,6 +155,25 @@ __device__ __forceinline__ void sym_block(const int lane, const T *__restrict__ 
   cs = (hf ? c2[1] : c2[0]) + __shfl_xor_sync(0xffffffffu, sc, 1);
 }
 
+// The power of two that brings a largest magnitude mx to [1, 2), and its
+// inverse.  The recurrences form u.Au, of third degree in the matrix; scaled
+// like this, which is exact, they take every matrix whose squares the QL
+// phase can form.
+template <class T> __device__ __forceinline__ void sym_scale(const T mx, T &to, T &back)
+{
+  const int lim = sizeof(T) == 8 ? 1000 : 120;
+  int k = 0;
+  if (mx > T(0) && mx < (T)INFINITY) k = max(-lim, min(lim, ilogb(mx)));
+  to = (T)ldexp(1.0, -k);
+  back = (T)ldexp(1.0, k);
+}
+template <class T> __device__ __forceinline__ T warp_max(T x)
+{
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x = fmax_t(x, __shfl_xor_sync(0xffffffffu, x, o));
+  return x;
+}
+
 // One step i (i = n-1 .. 1) removes column i with the reflector u whose raw
 // entries v are the rows < i of that column: u = v - anorm e_{i-1}, so
 //   A u = A v - anorm A e_{i-1},   u.A u = v.Av - 2 anorm (A v)_{i-1} + anorm^2 A_{i-1,i-1},
@@ -203,6 +222,7 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
   };
 
   // ---- blocks of this warp ----
+  T mx = T(0);  // largest magnitude
   T S[RS][32];
   int bR[RS], bC[RS];  // block rows and columns of the register slots
 #pragma unroll
@@ -221,6 +241,8 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
       S[s][x] = g < nblk ? elem(32 * bR[s] + 2 * lr + 8 * ((x >> 3) ^ xj) + ((x >> 2) & 1),
                                 32 * bC[s] + 2 * lc + 16 * (((x >> 1) & 1) ^ xh) + (x & 1))
                          : T(0);
+#pragma unroll
+    for (int x = 0; x < 32; x++) mx = fmax_t(mx, fabs_t(S[s][x]));
   }
   for (int l = RS * NW + warp; l < nl; l += NW) {
     const int g = l * CN + rank;
@@ -232,7 +254,9 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
 #pragma unroll
     for (int x = 0; x < 16; x++) {
       const int rr = 32 * r + 2 * lr + 8 * ((x >> 2) ^ xj) + ((x >> 1) & 1), cl = 32 * c + 2 * lc + 16 * ((x & 1) ^ xh);
-      sst2(B + (x * 32 + lane) * 2, elem(rr, cl), elem(rr, cl + 1));
+      const T a0 = elem(rr, cl), a1 = elem(rr, cl + 1);
+      sst2(B + (x * 32 + lane) * 2, a0, a1);
+      mx = fmax_t(mx, fmax_t(fabs_t(a0), fabs_t(a1)));
     }
   }
   for (int r = t; r < nr; r += NT) {
@@ -243,7 +267,35 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
   if (first && rank == 0 && t == 0) e_out[n - 1] = T(0);
   if (t < 8) sc[t] = T(0);
   for (int q = t; q < 64; q += NT) dotp[q] = T(0);  // and sg
-  if (CN > 1) cg::this_cluster().sync();
+  // scale: the largest magnitude of the CTA, then of the cluster's CTAs
+  mx = warp_max(mx);
+  if (lane == 0) prow[warp] = mx;  // prow is free until the first pass
+  __syncthreads();
+  mx = T(0);
+  for (int q = 0; q < NW; q++) mx = fmax_t(mx, prow[q]);
+  if (CN > 1) {
+    if (t < CN) *cg::this_cluster().map_shared_rank(dg + rank, t) = mx;
+    cg::this_cluster().sync();
+    mx = T(0);
+    for (int q = 0; q < CN; q++) mx = fmax_t(mx, dg[q]);
+  }
+  T to, back;
+  sym_scale(mx, to, back);
+#pragma unroll
+  for (int s = 0; s < RS; s++)
+#pragma unroll
+    for (int x = 0; x < 32; x++) S[s][x] *= to;
+  for (int l = RS * NW + warp; l < nl && l * CN + rank < nblk; l += NW) {
+    T *B = blk + (size_t)(l - RS * NW) * 1024 + 2 * lane;
+#pragma unroll
+    for (int x = 0; x < 16; x++) {
+      T a0, a1;
+      sld2(B + x * 64, a0, a1);
+      sst2(B + x * 64, a0 * to, a1 * to);
+    }
+  }
+  for (int r = t; r < nr; r += NT) cb[((n - 1) & 1) * nr + r] *= to;
+  if (CN > 1) cg::this_cluster().sync();  // also: dg is free for the first step's sums
   else __syncthreads();
 
   for (int i = n - 1;; --i) {
@@ -315,7 +367,7 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
         w = fma(alpha, u, beta * fma(-anorm, c, y));
         const T x = fma(w, ul, fma(u, wi, c));
         if (r == i) {
-          if (rank == 0 && i >= stop) d_out[i] = x;
+          if (rank == 0 && i >= stop) d_out[i] = x * back;
         } else {
           v = x;
         }
@@ -339,7 +391,7 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
         for (int x = 0; x < 32; x++) {
           const int r = 2 * lr + 8 * ((x >> 3) ^ xj) + ((x >> 2) & 1), c = 2 * lc + 16 * (((x >> 1) & 1) ^ xh) + (x & 1);
           const T v = fma(xR[32 + r], xC[c], fma(xR[r], xC[32 + c], get(x)));
-          if (32 * R + r <= 32 * C + c) A[32 * R + r + (size_t)(32 * C + c) * nm] = v;
+          if (32 * R + r <= 32 * C + c) A[32 * R + r + (size_t)(32 * C + c) * nm] = v * back;
         }
       };
       const int nout = (stop / 32) * (stop / 32 + 1) / 2;
@@ -375,7 +427,7 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
         sc[1] = b;
         sc[2] = l;
         if (rank == 0) {
-          e_out[i - 1] = an;
+          e_out[i - 1] = an * back;
           beta_out[i] = (double)b;
         }
       }

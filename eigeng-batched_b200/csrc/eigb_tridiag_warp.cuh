@@ -50,7 +50,26 @@ __device__ void tridiag_warp(T *A, const int nm, const int n, const T *Ap, T *d_
           const int a = min(r, c), b = max(r, c);
           S[j][e][h][f] = b < n ? V[b * TW_LD + a] : T(0);
         }
-  T col = lane < n ? V[(n - 1) * TW_LD + lane] : T(0);  // raw column i of the matrix before the pending update
+  T mx = T(0);
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int f = 0; f < 2; f++) mx = fmax_t(mx, fabs_t(S[j][e][h][f]));
+  T to, back;
+  sym_scale(warp_max(mx), to, back);
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int f = 0; f < 2; f++) S[j][e][h][f] *= to;
+  T col = lane < n ? V[(n - 1) * TW_LD + lane] * to : T(0);  // raw column i of the matrix before the pending update
   __syncwarp();
   uwv[lane] = uwv[32 + lane] = uwv[64 + lane] = T(0);
 
@@ -66,7 +85,7 @@ __device__ void tridiag_warp(T *A, const int nm, const int n, const T *Ap, T *d_
     const T u = lane == i ? ul : (lane < i ? v : T(0));
     const T w = lane <= i ? fma(alpha, u, beta * fma(-anorm, col, y)) : T(0);
     const T x = fma(w, ul, fma(u, wi, col));
-    if (lane == i) d_out[i] = x;
+    if (lane == i) d_out[i] = x * back;
     if (i < n - 1) V[(i + 1) * TW_LD + lane] = u;
     v = lane < i ? x : T(0);
     if (i == 0) break;
@@ -81,7 +100,7 @@ __device__ void tridiag_warp(T *A, const int nm, const int n, const T *Ap, T *d_
     ul = last - anorm;
     beta = T(1) / flip0to1(ul * anorm);
     if (lane == 0) {
-      e_out[i - 1] = anorm;
+      e_out[i - 1] = anorm * back;
       beta_s[i] = beta;
     }
     // update with (u, w), product with v, column i-1
