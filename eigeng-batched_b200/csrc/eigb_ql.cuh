@@ -74,6 +74,14 @@ __host__ __device__ __forceinline__ Tql2Step<T> tql2_end(const Tql2Pre<T> &a, co
   k.sn = mul_rn(ei, a.y);
   k.r = mul_rn(a.sig, a.y);
   k.pn = mul_rn(a.y, a.q);
+  return k;
+}
+// the whole step, for p and e of any size
+template <class T>
+__host__ __device__ __forceinline__ Tql2Step<T> tql2_any(const T c, const T p, const T ei, const T di)
+{
+  const Tql2Pre<T> a = tql2_begin(c, p, ei, di);
+  Tql2Step<T> k = tql2_end(a, p, ei, di);
   if (!rsq_plain(a.sig)) {
     givens_any(p, ei, k.cn, k.sn, k.r);
     k.pn = fma(k.cn, di, -mul_rn(k.sn, k.gg));
@@ -211,7 +219,7 @@ __host__ __device__ int ql_tql2(QLGen<T> &g, const DEView<T> v, const int n, Rec
             g.s2 = g.s;
             const T ei = v.E(i);
             const T di = (i >= g.l + 2) ? v.D(i) - g.delta : v.D(i);
-            const Tql2Step<T> k = tql2_end(tql2_begin(g.c, g.p, ei, di), g.p, ei, di);
+            const Tql2Step<T> k = tql2_any(g.c, g.p, ei, di);
             g.p = k.pn;
             v.E(i + 1) = tql2_e1(k, g.s);
             v.D(i + 1) = tql2_d1(k, di);
@@ -398,17 +406,44 @@ template <class T> struct DEPair {
   __host__ __device__ __forceinline__ void put_e(const Cur &c, int k, T y) const { c[k * st].y = y; }
 };
 
+// Magnitude as an integer that orders as the magnitude does (the upper word
+// of a double), and bounds that keep p^2 + e^2 plain (rsq_plain) for every p:
+// |e| >= QL_LOW, and d, e of the whole matrix at most ql_high.
+__host__ __device__ __forceinline__ int ql_mag(double x)
+{
+#ifdef __CUDA_ARCH__
+  return __double2hiint(x) & 0x7fffffff;
+#else
+  long long b;
+  memcpy(&b, &x, 8);
+  return (int)(b >> 32) & 0x7fffffff;
+#endif
+}
+__host__ __device__ __forceinline__ int ql_mag(float x)
+{
+#ifdef __CUDA_ARCH__
+  return __float_as_int(x) & 0x7fffffff;
+#else
+  int b;
+  memcpy(&b, &x, 4);
+  return b & 0x7fffffff;
+#endif
+}
+template <class T> __host__ __device__ constexpr int ql_low() { return sizeof(T) == 8 ? 0x23000000 : 0x27000000; }  // 2^-463, 2^-49
+template <class T> __host__ __device__ constexpr int ql_high() { return sizeof(T) == 8 ? 0x5b700000 : 0x53000000; } // 2^440, 2^39
+
 // The rotation loop is bound by the latency of its recurrence (p -> y -> p)
 // and, with several chains a scheduler, by instruction issue.  What a
 // rotation leaves behind (its record, d and e of i+1) is therefore formed and
-// stored one step later, while that step's y is on its way, in one block
-// without branches but for rsq_plain's, and four steps are unrolled, which
-// turns the hand-over from step to step into register names.  Measured on
-// B200 against the loop that finished each rotation in place with the
-// library's rsqrt (phase 2, ms; not unrolled in brackets): FP64 n=128 L=4096
-// 2.44 -> 1.59 (1.80), n=256 L=2048 10.7 -> 6.4 (7.4), n=512 L=256 30.0 ->
-// 18.5 (21.2), n=1000 L=32 109 -> 67 (77); FP32 n=128 2.36 -> 1.11 (1.27),
-// n=256 9.2 -> 4.3 (5.0).
+// stored one step later, while that step's y is on its way, and four steps
+// are unrolled into one block without branches: whether every rotation of a
+// sweep will be plain is known before it, from the smallest |e| that the sweep
+// before left and the largest entry of the matrix.  (A test in each rotation
+// cost a quarter: it cut the block.)  Measured on B200 against the loop that
+// finished each rotation in place with the library's rsqrt (phase 2, ms; with
+// a test per rotation in brackets): FP64 n=128 L=4096 2.44 -> 1.30 (1.59),
+// n=256 L=2048 10.7 -> 5.1 (6.4), n=512 L=256 30.0 -> 14.6 (18.4), n=1000 L=32
+// 109 -> 53 (67); FP32 n=128 2.36 -> 0.87 (1.05), n=256 9.2 -> 3.2 (4.3).
 template <class T, class S>
 __host__ __device__ int ql_tql2_fast_s(const S v, const int n, Rec<T> *__restrict__ out, const int cap,
                                        const int max_sweep, int *ierr)
@@ -419,6 +454,15 @@ __host__ __device__ int ql_tql2_fast_s(const S v, const int n, Rec<T> *__restric
   *ierr = 0;
   if (n <= 1) return 0;
   T shift = T(0), tst1 = T(0);
+  bool small = true;  // no entry above ql_high (none is a NaN)
+  {
+    Cur q = v.at(0);
+    for (int i = 0; i < n; i++, v.move(q, 1)) {
+      T d0, e0;
+      v.get(q, 0, d0, e0);
+      small = small && ql_mag(d0) <= ql_high<T>() && ql_mag(e0) <= ql_high<T>();
+    }
+  }
   for (int l = 0; l < n; l++) {
     const Cur lp = v.at(l);
     {
@@ -448,6 +492,9 @@ __host__ __device__ int ql_tql2_fast_s(const S v, const int n, Rec<T> *__restric
     }
     if (m != l) {
       const int len = m - l;
+      // smallest |e| of the block: those found by the search are above tst1
+      int emin = ql_mag(tst1);
+      const bool above = small && emin >= ql_low<T>();
       int itr;
       for (itr = 0; itr < max_sweep; itr++) {
         if (nrec + 1 + len > cap) return -1;
@@ -474,29 +521,71 @@ __host__ __device__ int ql_tql2_fast_s(const S v, const int n, Rec<T> *__restric
         Rec<T> *o = out + nrec;
         T d_n, e_n;  // the next step's d(i), e(i), loaded a step ahead
         v.get(qp, -1, d_n, e_n);
+        // With every |e| of the block at least ql_low no rotation needs
+        // checking; e(l+1) .. e(m-1) of the next sweep are measured here, e(l)
+        // stays above tst1.
+        const bool fast = above && emin >= ql_low<T>();
+        emin = 0x7fffffff;
+        if (fast) {
+          auto step = [&](const bool first, const T sub, const bool more, const bool meas) {
+            c3 = c2;
+            c2 = c;
+            s2 = s;
+            ei = e_n;
+            const T dn = d_n - sub;
+            if (more) v.get(qp, -2, d_n, e_n);
+            const Tql2Pre<T> a = tql2_begin(c, p, ei, dn);
+            const T e1 = tql2_e1(k, so), d1 = tql2_d1(k, di);
+            Rec<T> rec;
+            rec.c = c;
+            rec.s = s;
+            *o++ = rec;
+            if (!first) v.put(qp, 1, d1, e1);
+            if (meas) emin = min(emin, ql_mag(e1));
+            k = tql2_end(a, p, ei, dn);
+            di = dn;
+            so = s;
+            p = k.pn;
+            c = k.cn;
+            s = k.sn;
+            v.move(qp, -1);
+          };
+          int i = m - 1;
+          step(true, i >= l + 2 ? delta : T(0), i > l, false);
+          i--;
+          if (i >= l) {
+            step(false, i >= l + 2 ? delta : T(0), i > l, false);
+            i--;
+          }
 #pragma unroll 4
-        for (int i = m - 1; i >= l; i--) {
-          c3 = c2;
-          c2 = c;
-          s2 = s;
-          ei = e_n;
-          const T dn = (i >= l + 2) ? d_n - delta : d_n;
-          v.get(qp, i > l ? -2 : -1, d_n, e_n);
-          const Tql2Pre<T> a = tql2_begin(c, p, ei, dn);
-          const T e1 = tql2_e1(k, so), d1 = tql2_d1(k, di);
-          Rec<T> rec;
-          rec.c = c;
-          rec.s = s;
-          *o++ = rec;
-          if (i < m - 1) v.put(qp, 1, d1, e1);
-          k = tql2_end(a, p, ei, dn);
-          di = dn;
-          so = s;
-          p = k.pn;
-          c = k.cn;
-          s = k.sn;
-          v.move(qp, -1);
+          for (; i >= l + 2; i--) step(false, delta, true, true);
+          for (; i >= l; i--) step(false, T(0), i > l, true);
+        } else {
+#pragma unroll 1
+          for (int i = m - 1; i >= l; i--) {
+            c3 = c2;
+            c2 = c;
+            s2 = s;
+            ei = e_n;
+            const T dn = (i >= l + 2) ? d_n - delta : d_n;
+            v.get(qp, i > l ? -2 : -1, d_n, e_n);
+            const T e1 = tql2_e1(k, so), d1 = tql2_d1(k, di);
+            Rec<T> rec;
+            rec.c = c;
+            rec.s = s;
+            *o++ = rec;
+            if (i < m - 1) v.put(qp, 1, d1, e1);
+            emin = min(emin, i < m - 2 ? ql_mag(e1) : 0x7fffffff);
+            k = tql2_any(c, p, ei, dn);
+            di = dn;
+            so = s;
+            p = k.pn;
+            c = k.cn;
+            s = k.sn;
+            v.move(qp, -1);
+          }
         }
+        if (len > 1) emin = min(emin, ql_mag(tql2_e1(k, so)));
         v.put(qp, 1, tql2_d1(k, di), tql2_e1(k, so));
         {
           Rec<T> rec;
