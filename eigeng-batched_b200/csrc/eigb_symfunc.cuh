@@ -18,7 +18,8 @@
 // B as it is loaded.
 //   n <= 32   one warp per matrix, fragments straight from global memory
 //   n <= 128  one CTA per matrix, a warp per tile: V is read once
-//   above     one CTA of 16 warps per 128 x 128 block of Z
+//   above     one CTA of 8 warps per 128 x 64 block of Z, two CTAs an SM
+// Panels keep the input's type; FP32 is widened as a fragment is loaded.
 #pragma once
 #include "eigb_common.cuh"
 
@@ -27,8 +28,9 @@ namespace eigb {
 enum { SYMF_DIAG = 0, SYMF_POW = 1, SYMF_EXP = 2 };
 
 constexpr int SF_KC = 16;     // columns of V per panel
-constexpr int SF_LD = 132;    // pitch of a panel: 4 mod 16 doubles, so that the fragment loads
-                              // (four columns, rows of 8) are free of bank conflicts
+// Pitch of a panel: 4 mod 16 doubles or 8 mod 32 floats, so that the fragment
+// loads (four columns, rows of 8) are free of bank conflicts.
+template <class T> __host__ __device__ constexpr int sf_ld() { return sizeof(T) == 8 ? 132 : 136; }
 
 template <class T> __device__ __forceinline__ T symf_apply(const int func, const T x, const T p)
 {
@@ -130,59 +132,74 @@ __global__ void __launch_bounds__(32 * SFW_WARPS) k_symfunc_w(const long L, cons
   sf_store<T>(z + (size_t)k * nm * n, nm, n, 0, 0, acc);
 }
 
-// n > 32: block (bi, bj) of 128 x 128 of one matrix per CTA.  MAXT = 320: one
-// block (n <= 128), a warp per tile on or above the diagonal; 512: 16 warps,
-// one per tile of the block, those below the diagonal idle.  Two panels of
-// SF_KC columns in flight; off the diagonal a panel holds the rows of both.
-__host__ __device__ inline size_t symf_smem_bytes(int n)
+// n > 32.  ONE (n <= 128): one CTA per matrix, a warp per tile on or above the
+// diagonal.  Else a CTA of 8 warps per block of 128 rows (bi) and 64 columns
+// (cj) that reaches the diagonal or lies above it, a warp per tile, those
+// below the diagonal idle.  Two panels of SF_KC columns in flight; one panel
+// holds the block's 128 rows and, unless they are among them, the rows of V
+// that its 64 columns take.
+// Nine loads from shared memory feed 16 mma, and each panel costs a barrier, so
+// warps in flight count; above 128 also the idle tiles of the blocks at the
+// diagonal and at the end (n=256: 18 TFLOP/s of the upper half).  Blocks of 128 x 64 with two CTAs an SM against
+// 128 x 128 with 16 warps and one, both types as doubles in the panel, B200,
+// ms: FP64 n=256 L=2048 2.18 / 1.87, n=512 L=256 1.85 / 1.59, n=1000 L=32
+// 1.66 / 1.43; FP32 n=128 L=4096 0.47 / 0.42, n=201 L=1000 0.87 / 0.68.
+template <class T> __host__ __device__ inline size_t symf_smem_bytes(int n)
 {
-  return sizeof(double) * 2 * (size_t)(n <= 128 ? 1 : 2) * SF_KC * SF_LD + sizeof(double) * (size_t)((n + 15) & ~15);
+  return sizeof(T) * 2 * (size_t)(n <= 128 ? 1 : 2) * SF_KC * sf_ld<T>() + sizeof(double) * (size_t)((n + 15) & ~15);
 }
-template <class T, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT == 320 ? 2 : 1) k_symfunc_tc(const int nm, const int n,
-                                                                         const T *__restrict__ v,
-                                                                         const T *__restrict__ w, T *__restrict__ z,
-                                                                         const int func, const T p, const int nblk)
+// column blocks of 64 of the row blocks before bi: those with 64 cj + 63 >= 128 b
+__host__ __device__ inline int symf_blocks(int n)
+{
+  const int nc = (n + 63) / 64, nb = (n + 127) / 128;
+  int t = 0;
+  for (int b = 0; b < nb; b++) t += nc - 2 * b;
+  return t;
+}
+template <class T, bool ONE>
+__global__ void __launch_bounds__(ONE ? 320 : 256, 2) k_symfunc_tc(const int nm, const int n, const T *__restrict__ v,
+                                                                   const T *__restrict__ w, T *__restrict__ z,
+                                                                   const int func, const T p, const int per)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr bool ONE = MAXT == 320;
-  const int per = ONE ? 1 : nblk * (nblk + 1) / 2;
+  constexpr int LD = sf_ld<T>();
   const long k = blockIdx.x / per;
-  int bi = 0, bj = 0;
-  if (!ONE) sf_tile((int)(blockIdx.x % per), bi, bj);
-  const bool two = bi != bj;
+  int bi = 0, cj = 0;
+  if (!ONE) {
+    int t = (int)(blockIdx.x % per);
+    const int nc = (n + 63) / 64;
+    while (t >= nc - 2 * bi) t -= nc - 2 * bi++;
+    cj = 2 * bi + t;
+  }
+  const bool two = !ONE && cj >= 2 * bi + 2;  // the columns' rows are not among the block's
   const T *V = v + (size_t)k * nm * n;
   const T *W = w + (size_t)k * n;
-  double *panel = reinterpret_cast<double *>(smem_raw);
-  constexpr int PS = (ONE ? 1 : 2) * SF_KC * SF_LD;
-  double *fw = panel + 2 * PS;
+  constexpr int PS = (ONE ? 1 : 2) * SF_KC * LD;
+  double *fw = reinterpret_cast<double *>(smem_raw);
+  T *panel = reinterpret_cast<T *>(fw + ((n + 15) & ~15));
   const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, warp = t >> 5, g = lane >> 2, q = lane & 3;
-  int ti, tj;
+  int ti, tj;  // tile in 32s
   if (ONE) {
     sf_tile(warp, ti, tj);
   } else {
-    ti = warp & 3;
-    tj = warp >> 2;
+    ti = 4 * bi + (warp & 3);
+    tj = 2 * cj + (warp >> 2);
   }
-  const int i0 = 128 * bi + 32 * ti, j0 = 128 * bj + 32 * tj;
+  const int i0 = 32 * ti, j0 = 32 * tj;
   const bool act = i0 <= j0 && j0 < n;
 
   for (int c = t; c < ((n + 15) & ~15); c += nt) fw[c] = c < n ? (double)symf_apply(func, W[c], p) : 0.0;
-  // panel of columns c0 .. c0+15: rows of the block rows bi (and bj)
-  auto fill = [&](const int c0, double *P) {
+  // panel of columns c0 .. c0+15: the block's rows (and its columns')
+  auto fill = [&](const int c0, T *P) {
     for (int h = 0; h < (two ? 2 : 1); h++) {
-      const int r0 = 128 * (h == 0 ? bi : bj);
-      const int rows = min(128, ((n - r0 + 31) & ~31));
+      const int r0 = h == 0 ? 128 * bi : 64 * cj;
+      const int rows = min(h == 0 ? 128 : 64, ((n - r0 + 31) & ~31));
       for (int c = warp; c < SF_KC; c += nt >> 5) {
-        double *D = P + (h * SF_KC + c) * SF_LD;
+        T *D = P + (h * SF_KC + c) * LD;
         const T *src = V + r0 + (size_t)(c0 + c) * nm;
         for (int r = lane; r < rows; r += 32) {
-          if (c0 + c < n && r0 + r < n) {
-            if (sizeof(T) == 8) cp_async<8>(D + r, src + r);
-            else D[r] = (double)src[r];
-          } else {
-            D[r] = 0.0;
-          }
+          if (c0 + c < n && r0 + r < n) cp_async<sizeof(T)>(D + r, src + r);
+          else D[r] = T(0);
         }
       }
     }
@@ -200,8 +217,8 @@ __global__ void __launch_bounds__(MAXT, MAXT == 320 ? 2 : 1) k_symfunc_tc(const 
     __syncthreads();
     if (c0 + SF_KC < n) fill(c0 + SF_KC, panel + (cur ^ 1) * PS);
     if (act) {
-      const double *PA = panel + cur * PS + q * SF_LD + 32 * ti + g;
-      const double *PB = panel + cur * PS + (two ? SF_KC * SF_LD : 0) + q * SF_LD + 32 * tj + g;
+      const T *PA = panel + cur * PS + q * LD + i0 - 128 * bi + g;
+      const T *PB = panel + cur * PS + q * LD + g + (two ? SF_KC * LD + j0 - 64 * cj : j0 - 128 * bi);
       const bool diag = i0 == j0;
 #pragma unroll
       for (int s = 0; s < SF_KC / 4; s++) {
@@ -209,8 +226,8 @@ __global__ void __launch_bounds__(MAXT, MAXT == 320 ? 2 : 1) k_symfunc_tc(const 
         const double f = fw[c0 + 4 * s + q];
 #pragma unroll
         for (int x = 0; x < 4; x++) {
-          a[x] = PA[4 * s * SF_LD + 8 * x];
-          b[x] = f * PB[4 * s * SF_LD + 8 * x];
+          a[x] = (double)PA[4 * s * LD + 8 * x];
+          b[x] = f * (double)PB[4 * s * LD + 8 * x];
         }
 #pragma unroll
         for (int y = 0; y < 4; y++)

@@ -2324,16 +2324,16 @@ cudaError_t symfunc_run(long L, int nm, int n, const T *v, const T *w, T *z, int
                                                                                                 (T)p);
     return cudaGetLastError();
   }
-  const int nblk = (n + 127) / 128, nb = (n + 31) / 32;
-  const long blocks = nblk == 1 ? L : L * nblk * (nblk + 1) / 2;
+  const int nb = (n + 31) / 32, per = n <= 128 ? 1 : symf_blocks(n);
+  const long blocks = L * per;
   if (blocks > 0x7fffffffL) return cudaErrorInvalidValue;
-  const size_t smem = symf_smem_bytes(n);
+  const size_t smem = symf_smem_bytes<T>(n);
   cudaError_t err = cudaSuccess;
-  if (nblk == 1) {
-    k_symfunc_tc<T, 320><<<(unsigned)blocks, 32 * nb * (nb + 1) / 2, smem, stream>>>(nm, n, v, w, z, func, (T)p, nblk);
+  if (n <= 128) {
+    k_symfunc_tc<T, true><<<(unsigned)blocks, 32 * nb * (nb + 1) / 2, smem, stream>>>(nm, n, v, w, z, func, (T)p, per);
   } else {
-    if ((err = set_smem(k_symfunc_tc<T, 512>, smem)) != cudaSuccess) return err;
-    k_symfunc_tc<T, 512><<<(unsigned)blocks, 512, smem, stream>>>(nm, n, v, w, z, func, (T)p, nblk);
+    if ((err = set_smem(k_symfunc_tc<T, false>, smem)) != cudaSuccess) return err;
+    k_symfunc_tc<T, false><<<(unsigned)blocks, 256, smem, stream>>>(nm, n, v, w, z, func, (T)p, per);
   }
   return cudaGetLastError();
 }

@@ -1,5 +1,5 @@
 """V f(w) V^T at the edges of its forms: one warp per matrix up to n = 32, a
-warp per 32 x 32 tile up to n = 128, 128 x 128 blocks above; orders that are
+warp per 32 x 32 tile up to n = 128, 128 x 64 blocks above; orders that are
 no multiple of the mma tiles or of the 16-column panels.
 
 Against the product in FP64: a term is rounded once when f(w_k) scales it and
@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", ["f64", "f32"])
 @pytest.mark.parametrize("n,nm,L", [(1, 1, 9), (2, 3, 5), (31, 31, 6), (32, 33, 3), (33, 33, 2), (47, 48, 3), (63, 63, 2),
-                                    (96, 96, 2), (97, 99, 2), (127, 127, 2), (129, 129, 2), (160, 161, 2), (255, 255, 2),
+                                    (96, 96, 2), (97, 99, 2), (127, 127, 2), (129, 129, 2), (160, 161, 2), (191, 191, 2), (193, 193, 2), (255, 255, 2),
                                     (257, 257, 1), (1024, 1024, 1)])
 def test_tiles(dtype, n, nm, L):
     import eigeng_b200 as E
