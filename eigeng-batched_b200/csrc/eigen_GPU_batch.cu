@@ -400,7 +400,8 @@ template <class T> size_t sym_smem(int n, const SymCfg &c)
 // launch with fewer CTAs or warps (0: none).  A matrix keeps its SMs to the
 // last step otherwise, and the last steps have little to do; where the batch
 // takes more than one wave of CTAs, another launch packs the small blocks
-// closer.  Measured on B200 (the reduction, ms, without / with): FP64 n=160
+// closer.  Measured on B200 (the reduction, ms, without / with): FP64 n=72
+// L=8000 1.96 / 1.78, n=96 L=8000 3.09 / 2.89, n=128 L=4096 3.05 / 2.81, n=160
 // L=3000 4.20 / 3.84, n=256 L=2048 9.68 / 8.39, n=512 L=256 14.0 / 10.3, n=1000
 // L=32 26.9 / 18.2; FP32 n=201 L=1000 1.57 / 1.37, n=512 L=256 6.80 / 5.30,
 // n=1000 L=32 14.1 / 9.3.  In a single wave it costs: FP64 n=512 L=32 1.76 /
@@ -408,7 +409,7 @@ template <class T> size_t sym_smem(int n, const SymCfg &c)
 template <class T> int sym_next(int n, long cnt, const SymCfg &c, int sms)
 {
   if (cnt * c.cn <= (long)sms * c.mb) return 0;
-  const int at64[] = {736, 512, 352, 256, 128, 0}, at32[] = {736, 512, 384, 160, 0};
+  const int at64[] = {736, 512, 352, 256, 128, 64, 0}, at32[] = {736, 512, 384, 160, 0};
   const int *at = sizeof(T) == 8 ? at64 : at32;
   while (*at >= n) at++;
   return *at;

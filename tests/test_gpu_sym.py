@@ -88,3 +88,24 @@ def test_packed_input_and_special_matrices(oracle_mod, dtype, n):
     scale = torch.linalg.matrix_norm(a0[ok].double()).clamp(min=1e-30)
     # n - 1 reflections and about n rotations per row and column
     assert (orth <= 32 * n * eps).all() and (torch.linalg.matrix_norm(R) / scale <= 32 * n * eps).all()
+
+
+@pytest.mark.parametrize("dtype,n,L", [("f64", 65, 900), ("f64", 96, 900), ("f64", 128, 460), ("f64", 129, 300),
+                                       ("f64", 353, 60), ("f32", 161, 310), ("f32", 385, 80)])
+def test_more_than_a_wave_of_matrices(dtype, n, L):
+    """Batches of more than one wave of CTAs hand their leading blocks over to
+    launches of smaller CTAs; every matrix still comes back as Q T Q^T."""
+    import eigeng_b200 as E
+    dt = torch.float64 if dtype == "f64" else torch.float32
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    x = (torch.rand((L, n, n), generator=g, device="cuda", dtype=torch.float64) * 2 - 1).to(dt)
+    A = (x.tril() + x.tril(-1).mT).double()
+    a = x.tril() + torch.full_like(x, float("nan")).triu(1)
+    d, e = _reduce(E, a, n, n)
+    T = torch.diag_embed(d) + torch.diag_embed(e[:, :n - 1], 1) + torch.diag_embed(e[:, :n - 1], -1)
+    Qt = a.double()
+    eps = torch.finfo(dt).eps
+    res = torch.linalg.matrix_norm(Qt.mT @ T @ Qt - A) / torch.linalg.matrix_norm(A)
+    orth = torch.linalg.matrix_norm(Qt @ Qt.mT - torch.eye(n, dtype=torch.float64, device="cuda")) / n ** 0.5
+    assert res.max().item() <= 8 * n * eps and orth.max().item() <= 8 * n * eps, (res.max(), orth.max())
