@@ -313,10 +313,16 @@ cudaError_t buffer_size(long L, int nm, int n, int m, size_t *lwork, const eigen
   return cudaSuccess;
 }
 
+// Admits a launch of kern with that much dynamic shared memory.  The limit set
+// is the same for every size (227 KB less the static shared memory of any
+// kernel here), so that of two threads whose calls launch one kernel at
+// different orders neither lowers the other's limit before its launch.  (A
+// constant of sm_100: asking the device costs 3 us a call.)
 template <class K> cudaError_t set_smem(K kern, size_t bytes)
 {
-  if (bytes <= 46 * 1024) return cudaSuccess;  // 48 KB less the static shared memory of any kernel here
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  constexpr size_t fixed = 2 * 1024, all = 227 * 1024 - fixed;
+  if (bytes <= 48 * 1024 - fixed) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(bytes, all));
 }
 
 // FP32 phase 1 in registers for 32 < n <= 64 (2 x 2 blocks of 32 x 32).  In

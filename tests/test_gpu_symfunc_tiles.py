@@ -36,3 +36,41 @@ def test_tiles(dtype, n, nm, L):
         tol = 2 * (n + 2) * e64 * mag + (4 * e * mag if dtype == "f32" else 8 * e64 * mag) + e * ref.abs()
         assert ((got - ref).abs() <= tol).all()
         assert torch.equal(got, got.mT) and torch.isnan(z[:, :, n:]).all()
+
+
+def test_threads_of_different_orders():
+    """Two host threads that launch the same kernels at different orders, each
+    on its own stream: every call succeeds and gives the bits of a lone one."""
+    import threading
+    import eigeng_b200 as E
+    out, errors = {}, []
+
+    def work(n, reps):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                g = torch.Generator(device="cuda")
+                g.manual_seed(n)
+                v = torch.randn((2, n, n), generator=g, device="cuda", dtype=torch.float64)
+                w = torch.rand((2, n), generator=g, device="cuda", dtype=torch.float64)
+                a0 = v + v.mT
+                for _ in range(reps):
+                    z = torch.empty_like(v)
+                    E.symfunc(v, w, n, E.FUNC_DIAG, 0.0, n, z)
+                    a = a0.clone()
+                    ev, info = E.solve(a, n)
+                torch.cuda.current_stream().synchronize()
+                out[n, reps] = (z, a, ev)
+        except Exception as e:  # noqa: BLE001
+            errors.append((n, repr(e)))
+
+    orders = (200, 250)  # one kernel in each phase, other sizes of shared memory
+    for n in orders:
+        work(n, 1)
+    threads = [threading.Thread(target=work, args=(n, 150)) for n in orders]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for n in orders:
+        assert all(torch.equal(x, y) for x, y in zip(out[n, 1], out[n, 150]))
