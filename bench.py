@@ -225,6 +225,14 @@ def measured_traffic(kernel, dtype, n):
     return None
 
 
+def solve_launches(n, dtype, method):
+    """Kernels of one plain solve of one chunk, at least: a reduction that
+    hands its leading blocks over to smaller CTAs adds one launch for each."""
+    if n <= 32 or (dtype == "f32" and n <= 64):
+        return 1 if method == "jacobi" and n <= 32 else 3
+    return 6 if n >= 128 else 5  # k1_sym, k1_factor, k1_formq, k2_ql, k3_wave + k3_cta or k3_tmem
+
+
 def alg_bytes(n, esize):
     """Compulsory bytes per matrix: read A, write V and w."""
     return esize * (2 * n * n + n)
@@ -875,7 +883,7 @@ def main():
         "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
         "dtype": args.dtype, "data": "synthetic, seeded on device: " + FAMILY_TEXT[args.family],
         "config": workload_config(args, world, l2_note),
-        "gpu_launches": 3 * nchunks * args.steps,
+        "gpu_launches": solve_launches(n, args.dtype, args.method) * nchunks * args.steps,
         "correctness": {"reference_gate_flags": gate_fail, "info_nonzero": info_fail,
                         "max_err1": float(e1.max().item()), "max_err2": float(e2.max().item())},
         "phases_ms": {k: float(v) for k, v in zip(names, ph)},
