@@ -270,7 +270,10 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
   // scale: the largest magnitude of the CTA, then of the cluster's CTAs
   mx = warp_max(mx);
   if (lane == 0) prow[warp] = mx;  // prow is free until the first pass
-  __syncthreads();
+  // A CTA's shared memory may be written by another only once it runs: the
+  // cluster meets before the first such store.
+  if (CN > 1) cg::this_cluster().sync();
+  else __syncthreads();
   mx = T(0);
   for (int q = 0; q < NW; q++) mx = fmax_t(mx, prow[q]);
   if (CN > 1) {

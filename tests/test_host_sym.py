@@ -1,0 +1,90 @@
+"""The reductions of phase 1 on chip (k1_sym, k1_warp), run on the CPU from
+the library's source: fibers for the GPU threads, barriers and shuffles of
+warps, CTAs and clusters (tests/host/simt.hpp).  Its schedule lets one CTA of a
+cluster go as far as it can before the next one starts."""
+import ctypes
+import os
+import subprocess
+import tempfile
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+HOST = os.path.join(ROOT, "tests", "host")
+CUDA = "/usr/local/cuda/include"
+
+F64, F32 = np.float64, np.float32
+
+
+@pytest.fixture(scope="module")
+def lib():
+    if not os.path.exists(os.path.join(CUDA, "cuda_runtime.h")):
+        pytest.skip("CUDA headers not available")
+    out = os.path.join(tempfile.mkdtemp(prefix="eigb_sym_"), "libsym_host.so")
+    subprocess.check_call(["g++", "-x", "c++", "-std=c++20", "-O1", "-ffp-contract=off", "-Wno-unknown-pragmas", "-fPIC",
+                           "-U_FORTIFY_SOURCE",  # it takes jumps between stacks for an error
+                           "-shared", "-I" + CUDA, "-o", out, os.path.join(HOST, "sym_host.cu")])
+    so = ctypes.CDLL(out)
+    P, I = ctypes.c_void_p, ctypes.c_int
+    for s in ("d", "f"):
+        f = getattr(so, "host_sym_" + s)
+        f.restype, f.argtypes = ctypes.c_long, [I, I, I, P, I, I, I, I, P, P, P, P, I, P, I]
+    return so
+
+
+def _p(x):
+    return None if x is None else ctypes.c_void_p(x.ctypes.data)
+
+
+def uniform(n, dtype, seed):
+    b = np.random.default_rng(seed).uniform(-1, 1, (n, n))
+    return ((b + b.T) / 2).astype(dtype)
+
+
+def launch(lib, form, A, m, stop, first, d, e, V, beta, high_first=0):
+    """One launch; the number of accesses to CTAs that were not running."""
+    f = lib.host_sym_d if A.dtype == F64 else lib.host_sym_f
+    r = f(*form, _p(A), A.shape[1], m, stop, first, None, _p(d), _p(e), _p(V), V.shape[1], _p(beta), high_first)
+    assert r >= 0, "a thread waits for good" if r == -1 else "form not built"
+    return r
+
+
+def reflectors(V, beta):
+    """Q = (H_1 ... H_{n-1})^T from reflector k in V[k, :k]."""
+    n = V.shape[0]
+    Q = np.eye(n)
+    for k in range(1, n):
+        v = np.zeros(n)
+        v[:k] = V[k, :k]
+        Q = Q + beta[k] * np.outer(Q @ v, v)
+    return Q.T
+
+
+def tridiagonal(d, e):
+    e = e.astype(F64)
+    return np.diag(d.astype(F64)) + np.diag(e[:-1], 1) + np.diag(e[:-1], -1)
+
+
+def reduce(lib, form, a0, high_first=0):
+    n, dt = a0.shape[0], a0.dtype
+    A, V = a0.copy(), np.full((n, (n + 7) & ~7), np.nan, dt)
+    d, e, beta = np.full(n, np.nan, dt), np.full(n, np.nan, dt), np.full(n, np.nan)
+    early = launch(lib, form, A, n, 0, 1, d, e, V, beta, high_first)
+    return early, d, e, reflectors(V, beta)
+
+
+@pytest.mark.parametrize("high_first", [0, 1])
+@pytest.mark.parametrize("dtype,form,n", [(F64, (8, 2, 2), 70), (F64, (8, 2, 4), 70), (F64, (8, 2, 8), 40),
+                                          (F64, (8, 2, 16), 40), (F32, (8, 4, 2), 70), (F32, (8, 4, 4), 40),
+                                          (F32, (8, 4, 8), 40)])
+def test_cluster_touches_only_running_ctas(lib, dtype, form, n, high_first):
+    """Shared memory of another CTA may be accessed only once all CTAs of the
+    cluster run, and until they end; and A = Q T Q^T."""
+    a0 = uniform(n, dtype, n)
+    early, d, e, Q = reduce(lib, form, a0, high_first)
+    assert early == 0
+    eps = np.finfo(dtype).eps
+    a = a0.astype(F64)
+    assert np.linalg.norm(Q @ tridiagonal(d, e) @ Q.T - a) <= 8 * n * eps * np.linalg.norm(a)
+    assert np.linalg.norm(Q.T @ Q - np.eye(n)) <= 8 * n * eps * n ** 0.5
