@@ -137,18 +137,28 @@ __global__ void k_n1(const KP<T> p)
 }
 
 // ---------------------------------------------------------------- phase 1
+template <class T, bool SCALED>
+__device__ __forceinline__ bool k1_warp_run(const KP<T> &p, const long k, unsigned char *smem)
+{
+  return tridiag_warp<T, SCALED>(mat_ptr(p, k), p.nm, p.n, p.ap ? p.ap + (size_t)k * packed_size(p.n) : nullptr,
+                                 p.d + k * p.n, p.e + k * p.n,
+                                 reinterpret_cast<T *>(smem) + (threadIdx.x >> 5) * tw_smem_elems());
+}
+template <class T> __device__ __noinline__ void k1_warp_again(const KP<T> &p, const long k, unsigned char *smem)
+{
+  k1_warp_run<T, true>(p, k, smem);
+}
 // Bound by instruction issue and the steps' exchanges, so by warps in
 // flight: registers bounded for four CTAs an SM (five, with spills, 0.71 ms).
 // B200, n=32 FP64 L=16384: 0.40 ms, the matrix in shared memory 0.66.
 template <class T>
-__global__ void __launch_bounds__(32 * K1W_NW, 4) k1_warp(const KP<T> p)
+__global__ void __launch_bounds__(32 * K1W_NW, 4) k1_warp(const __grid_constant__ KP<T> p)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int wid = threadIdx.x >> 5;
   const long k = (long)blockIdx.x * K1W_NW + wid;
   if (k >= p.Lc) return;  // uniform per warp; no CTA barrier is used below
-  tridiag_warp<T>(mat_ptr(p, k), p.nm, p.n, p.ap ? p.ap + (size_t)k * packed_size(p.n) : nullptr, p.d + k * p.n,
-                  p.e + k * p.n, reinterpret_cast<T *>(smem_raw) + wid * tw_smem_elems());
+  if (k1_warp_run<T, false>(p, k, smem_raw)) k1_warp_again<T>(p, k, smem_raw);
 }
 
 // Shared-memory elements of k1_cta: red[72], beta[n], pv[n],
@@ -255,19 +265,36 @@ __global__ void __launch_bounds__(32 * SPLIT, 1024 / (32 * SPLIT)) k1_cl(const K
                                reinterpret_cast<T *>(smem_raw));
 }
 
+template <class T, int NW, int RS, int CN, bool SCALED>
+__device__ __forceinline__ bool k1_sym_run(const KP<T> &p, const long k, const int m, const int stop,
+                                           unsigned char *smem)
+{
+  unsigned char *v = p.vw + (size_t)k * p.vstride;
+  return tridiag_sym<T, NW, RS, CN, SCALED>(
+      mat_ptr(p, k), p.nm, m, stop, m == p.n, p.ap && m == p.n ? p.ap + (size_t)k * packed_size(p.n) : nullptr,
+      p.d + k * p.n, p.e + k * p.n, reinterpret_cast<T *>(v + fq_off_v(p.n)), fq_ldv(p.n),
+      reinterpret_cast<double *>(v), reinterpret_cast<T *>(smem));
+}
+template <class T, int NW, int RS, int CN>
+__device__ __noinline__ void k1_sym_again(const KP<T> &p, const long k, const int m, const int stop,
+                                          unsigned char *smem)
+{
+  k1_sym_run<T, NW, RS, CN, true>(p, k, m, stop, smem);
+}
 // Reduction of k1_sym<T, NW, RS, CN>: NW warps, RS blocks of a warp in
 // registers, CN CTAs per matrix (see eigb_tridiag_sym.cuh and sym_cfg), of the
 // leading m x m block down to order `stop`.
 template <class T, int NW, int RS, int CN, int MB>
-__global__ void __launch_bounds__(32 * NW, MB) k1_sym(const KP<T> p, const int m, const int stop)
+__global__ void __launch_bounds__(32 * NW, MB) k1_sym(const __grid_constant__ KP<T> p, const int m, const int stop)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const long k = blockIdx.x / CN;
-  unsigned char *v = p.vw + (size_t)k * p.vstride;
-  tridiag_sym<T, NW, RS, CN>(mat_ptr(p, k), p.nm, m, stop, m == p.n,
-                             p.ap && m == p.n ? p.ap + (size_t)k * packed_size(p.n) : nullptr, p.d + k * p.n,
-                             p.e + k * p.n, reinterpret_cast<T *>(v + fq_off_v(p.n)), fq_ldv(p.n),
-                             reinterpret_cast<double *>(v), reinterpret_cast<T *>(smem_raw));
+  // The second run is a call in FP64 and inline in FP32: the other way round
+  // FP64 n=512 L=256 takes 1.8 % longer (spills), FP32 n=128 L=4096 1.6 %.
+  if (k1_sym_run<T, NW, RS, CN, false>(p, k, m, stop, smem_raw)) {
+    if (sizeof(T) == 4) k1_sym_run<T, NW, RS, CN, true>(p, k, m, stop, smem_raw);
+    else k1_sym_again<T, NW, RS, CN>(p, k, m, stop, smem_raw);
+  }
 }
 
 // Block factors of the formation of Q, one warp per (matrix, block).

@@ -155,17 +155,36 @@ __device__ __forceinline__ void sym_block(const int lane, const T *__restrict__ 
   cs = (hf ? c2[1] : c2[0]) + __shfl_xor_sync(0xffffffffu, sc, 1);
 }
 
-// The power of two that brings a largest magnitude mx to [1, 2), and its
-// inverse.  The recurrences form u.Au, of third degree in the matrix; scaled
-// like this, which is exact, they take every matrix whose squares the QL
-// phase can form.
-template <class T> __device__ __forceinline__ void sym_scale(const T mx, T &to, T &back)
+// Range.  The recurrences form u.Au, of third degree in the matrix, and
+// beta = 1 / (l anorm) of degree -2 in a column, so both ends of the exponent
+// range limit them.  Powers of two, which are exact, keep them inside:
+//  - the matrix is scaled so that its largest magnitude mx lies in
+//    [2^K, 2^(K+1)), K as large as the third-degree sums of n <= 1024 allow:
+//    they stay below 2^7 |A|^3 with |A| <= 2^10 mx, so 40 + 3 K < 1023 (127);
+//  - a column whose squares sum to less than sym_tiny, far below the rest of
+//    the matrix, has to be scaled to entries below 2 by itself.  From sym_tiny
+//    on |v|^3 is a normal number with all its bits (640 * 3/2 < 1022 - 53;
+//    66 * 3/2 < 126 - 24).  A reflector does not change with the length of
+//    its u; only the subdiagonal entry is scaled back.
+// So blocks of a matrix may differ by more than the square root of the range.
+// Scaled columns are rare and the test for them must precede the pass over
+// the matrix (1 to 3 % of the solve: n=12 70.6 -> 72.7 us, n=256 FP64 32.50 ->
+// 32.69 ms), so a first run only notes beside the pass whether it met one (70.0
+// us, 32.50 ms); a second run (SCALED) then starts from the input, which the
+// first has left alone.
+template <class T> __device__ __forceinline__ T sym_tiny() { return sizeof(T) == 8 ? (T)0x1p-640 : (T)0x1p-66; }
+// to: the power of two for a largest magnitude mx > 0 to reach [2^K, 2^(K+1)); back: its inverse
+template <class T> __device__ __forceinline__ void sym_pow2(const T mx, const int K, T &to, T &back)
 {
   const int lim = sizeof(T) == 8 ? 1000 : 120;
   int k = 0;
-  if (mx > T(0) && mx < (T)INFINITY) k = max(-lim, min(lim, ilogb(mx)));
+  if (mx > T(0) && mx < (T)INFINITY) k = max(-lim, min(lim, ilogb(mx) - K));
   to = (T)ldexp(1.0, -k);
   back = (T)ldexp(1.0, k);
+}
+template <class T> __device__ __forceinline__ void sym_scale(const T mx, T &to, T &back)
+{
+  sym_pow2(mx, sizeof(T) == 8 ? 300 : 28, to, back);
 }
 template <class T> __device__ __forceinline__ T warp_max(T x)
 {
@@ -192,10 +211,12 @@ template <class T> __device__ __forceinline__ T warp_max(T x)
 //
 // Reduces the leading n x n block of A down to order `stop` (0: to the end),
 // where it leaves the updated leading block in A's upper triangle for a call
-// with fewer warps or CTAs; `first` is the call on the whole matrix.
-template <class T, int NW, int RS, int CN>
-__device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, const bool first, const T *Ap, T *d_out,
-                            T *e_out, T *V, const int ldv, double *beta_out, T *sm)
+// with fewer warps or CTAs; `first` is the call on the whole matrix.  Returns
+// true if it has to be run again with SCALED; A is as it was then.
+template <class T, int NW, int RS, int CN, bool SCALED>
+__device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, const int stop, const bool first,
+                                            const T *Ap, T *d_out, T *e_out, T *V, const int ldv, double *beta_out,
+                                            T *sm)
 {
   constexpr int NT = 32 * NW;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -209,7 +230,7 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
   T *cb = uwv + 3 * nr;  // 2 * nr
   T *dotp = cb + 2 * nr; // 32
   T *sg = dotp + 32;     // 32
-  T *sc = sg + 32;       // 8: anorm, beta, ul
+  T *sc = sg + 32;       // 8: anorm, beta, ul, whether a column was tiny, the factor of a scaled column's e
   T *dg = sc + 8;        // 2 * CN
   T *yg = dg + (CN > 1 ? 2 * CN : 0);  // the CTAs' sums: 2 * CN * nr, or nr totals and home * CN * 32
   T *yh = yg + nr;
@@ -383,7 +404,9 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
     }
     if (i == 0) break;
     if (i < stop) {  // i = stop - 1: the pending update alone, and the block goes out
+      const bool again = sc[3] != T(0);
       __syncthreads();
+      if (again) return true;
       auto out = [&](const int l, auto get) {
         const int g = l * CN + rank;
         int C = 0;
@@ -405,11 +428,34 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
 #pragma unroll
       for (int s = 0; s < RS; s++)
         if ((s * NW + warp) * CN + rank < nout) out(s * NW + warp, [&](const int x) { return S[s][x]; });
-      return;
+      return false;
     }
     sig = warp_sum(sig);
     if (lane == 0) sg[warp] = sig;
     __syncthreads();
+    if constexpr (SCALED) {
+      T s = T(0), eb = T(1);
+      for (int q = 0; q < NW; q++) s += sg[q];
+      if (s < sym_tiny<T>()) {
+        T mv = T(0), up;
+        for (int r = t; r < nr; r += NT) mv = fmax_t(mv, fabs_t(uwv[96 * (r >> 5) + 64 + (r & 31)]));
+        mv = warp_max(mv);
+        if (lane == 0) dotp[warp] = mv;  // free until the end of the pass
+        __syncthreads();
+        for (int q = 0; q < NW; q++) mv = fmax_t(mv, dotp[q]);
+        sym_pow2(mv, 0, up, eb);
+        s = T(0);
+        for (int r = t; r < nr; r += NT) {
+          T *v = uwv + 96 * (r >> 5) + 64 + (r & 31);
+          *v *= up;
+          s = fma(*v, *v, s);
+        }
+        s = warp_sum(s);
+        if (lane == 0) sg[warp] = s;
+      }
+      if (t == 0) sc[4] = eb;
+      __syncthreads();
+    }
 
     // ---- the reflector's scalars, in the last warp ----
     if (warp == NW - 1) {
@@ -430,9 +476,15 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
         sc[1] = b;
         sc[2] = l;
         if (rank == 0) {
-          e_out[i - 1] = an * back;
+          e_out[i - 1] = (SCALED ? an * sc[4] : an) * back;
           beta_out[i] = (double)b;
         }
+      }
+      // l an is in [-2, -1] |v|^2; 0 for a v whose squares vanish, or no v
+      if (!SCALED && (b <= T(-1) / sym_tiny<T>() || b > T(0))) {
+        bool any = b < T(0);
+        for (int r = lane; r < i; r += 32) any |= uwv[3 * (r - lane) + 64 + lane] != T(0);
+        if (__any_sync(0xffffffffu, any) && lane == 0) sc[3] = T(1);
       }
     }
 
@@ -538,6 +590,9 @@ __device__ void tridiag_sym(T *A, const int nm, const int n, const int stop, con
     }
   }
   if (t == 0 && rank == 0) beta_out[0] = 0.0;
+  const bool again = sc[3] != T(0);
+  __syncthreads();  // a second run begins with its shared memory
+  return again;
 }
 
 }  // namespace eigb

@@ -18,8 +18,11 @@ constexpr int TW_LD = 34;  // pitch of the reflectors and of the staged matrix: 
 // shared-memory elements per warp: reflectors / staging, (u, w, v), column and product, beta
 __host__ __device__ constexpr int tw_smem_elems() { return 32 * TW_LD + 96 + 64 + 32; }
 
-template <class T>
-__device__ void tridiag_warp(T *A, const int nm, const int n, const T *Ap, T *d_out, T *e_out, T *sm)
+// Returns true, with A as it was, if it has to be run again with SCALED
+// (see eigb_tridiag_sym.cuh).
+template <class T, bool SCALED>
+__device__ __forceinline__ bool tridiag_warp(T *A, const int nm, const int n, const T *Ap, T *d_out, T *e_out,
+                                             T *sm)
 {
   const int lane = threadIdx.x & 31;
   const int lr = lane & 3, lc = lane >> 2, xj = lane >> 3;
@@ -94,13 +97,23 @@ __device__ void tridiag_warp(T *A, const int nm, const int n, const T *Ap, T *d_
     uwv[64 + lane] = v;
     __syncwarp();
     // the reflector's scalars
-    const T sig = warp_sum(v * v);
+    T sig = warp_sum(v * v), eb = T(1);  // eb: scales a scaled column's e back
+    if constexpr (SCALED) {
+      if (sig < sym_tiny<T>()) {
+        T up;
+        sym_pow2(warp_max(fabs_t(v)), 0, up, eb);
+        v *= up;
+        uwv[64 + lane] = v;
+        __syncwarp();
+        sig = warp_sum(v * v);
+      }
+    }
     const T last = __shfl_sync(0xffffffffu, v, i - 1);
     anorm = -copysign_t(sqr_t(sig), last);
     ul = last - anorm;
     beta = T(1) / flip0to1(ul * anorm);
     if (lane == 0) {
-      e_out[i - 1] = anorm * back;
+      e_out[i - 1] = anorm * eb * back;
       beta_s[i] = beta;
     }
     // update with (u, w), product with v, column i-1
@@ -155,6 +168,13 @@ __device__ void tridiag_warp(T *A, const int nm, const int n, const T *Ap, T *d_
   }
   if (lane == 0) e_out[n - 1] = T(0);
   __syncwarp();
+  if (!SCALED) {  // a tiny column, by its beta = 1 / (l an) as in tridiag_sym
+    const T b = lane > 0 && lane < n ? beta_s[lane] : T(-1);
+    bool tiny = b <= T(-1) / sym_tiny<T>();
+    if (b > T(0))
+      for (int r = 0; r < lane; r++) tiny |= V[lane * TW_LD + r] != T(0);
+    if (__any_sync(0xffffffffu, tiny)) return true;
+  }
 
   // M <- M + beta_k (M u_k) u_k^T, row r in lane r
   T M[32];
@@ -193,6 +213,7 @@ __device__ void tridiag_warp(T *A, const int nm, const int n, const T *Ap, T *d_
   __syncwarp();
   if (lane < n)
     for (int c = 0; c < n; c++) A[lane + (size_t)c * nm] = V[c * TW_LD + lane];
+  return false;
 }
 
 }  // namespace eigb

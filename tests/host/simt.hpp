@@ -25,8 +25,6 @@ namespace simt {
 struct Barrier {
   int need = 0, here = 0;
   long gen = 0;
-  unsigned bits = 0;       // and/or reductions: of the arrivals, and of the last round
-  bool all = true, last_all = true;
 };
 struct Fiber {
   ucontext_t ctx;  // its first entry; later switches by jumps, which make no system call
@@ -66,8 +64,6 @@ inline void block(Barrier &b)  // arrives; returns when all have
 {
   if (++b.here == b.need) {
     b.here = 0;
-    b.last_all = b.all;
-    b.all = true;
     b.gen++;
     return;
   }
@@ -178,15 +174,14 @@ struct NDim {
 #define blockDim (simt::NDim())
 template <class T> T __shfl_xor_sync(unsigned, T x, int o) { return simt::shfl(x, (simt::m->cur->tid & 31) ^ o); }
 template <class T> T __shfl_sync(unsigned, T x, int s) { return simt::shfl(x, s & 31); }
+inline int __any_sync(unsigned, int p)
+{
+  int any = 0;
+  for (int o = 0; o < 32; o++) any |= simt::shfl(p, o);
+  return any;
+}
 inline void __syncwarp() { simt::block(simt::cta().warps[simt::m->cur->tid >> 5].bar); }
 inline void __syncthreads() { simt::block(simt::cta().bar); }
-inline int __syncthreads_and(int p)
-{
-  simt::Barrier &b = simt::cta().bar;
-  b.all = b.all && p;
-  simt::block(b);
-  return b.last_all;
-}
 template <class T> T min(T a, T b) { return b < a ? b : a; }
 template <class T> T max(T a, T b) { return a < b ? b : a; }
 

@@ -13,7 +13,8 @@ static long sym(T *A, int nm, int m, int stop, bool first, const T *Ap, T *d, T 
 {
   const size_t bytes = sizeof(T) * eigb::sym_smem_elems(m, NW, RS, CN);
   return simt::run(CN, 32 * NW, bytes, high_first != 0, [&] {
-    eigb::tridiag_sym<T, NW, RS, CN>(A, nm, m, stop, first, Ap, d, e, V, ldv, beta, simt::shared<T>());
+    if (eigb::tridiag_sym<T, NW, RS, CN, false>(A, nm, m, stop, first, Ap, d, e, V, ldv, beta, simt::shared<T>()))
+      eigb::tridiag_sym<T, NW, RS, CN, true>(A, nm, m, stop, first, Ap, d, e, V, ldv, beta, simt::shared<T>());
   });
 }
 template <class T>
@@ -47,7 +48,18 @@ static long sym_any(int nw, int rs, int cn, T *A, int nm, int m, int stop, int f
   return -2;
 }
 
+// k1_warp for one matrix, n <= 32: Q (A = Q T Q^T) in A's place
+template <class T> static long warp(T *A, int nm, int n, const T *Ap, T *d, T *e)
+{
+  return simt::run(1, 32, sizeof(T) * eigb::tw_smem_elems(), false, [&] {
+    if (eigb::tridiag_warp<T, false>(A, nm, n, Ap, d, e, simt::shared<T>()))
+      eigb::tridiag_warp<T, true>(A, nm, n, Ap, d, e, simt::shared<T>());
+  });
+}
+
 extern "C" {
+long host_warp_d(double *A, int nm, int n, const double *Ap, double *d, double *e) { return warp(A, nm, n, Ap, d, e); }
+long host_warp_f(float *A, int nm, int n, const float *Ap, float *d, float *e) { return warp(A, nm, n, Ap, d, e); }
 long host_sym_d(int nw, int rs, int cn, double *A, int nm, int m, int stop, int first, const double *Ap, double *d,
                 double *e, double *V, int ldv, double *beta, int hf)
 {

@@ -25,7 +25,7 @@ def hostlibs():
     for name in ("ql_host", "tridiag_host", "apply_host"):
         out = os.path.join(td, f"lib{name}.so")
         subprocess.check_call([NVCC, "-O2", "-std=c++20", "-Xcompiler", "-fPIC", "-shared",
-                               "-Wno-deprecated-gpu-targets", "-diag-suppress", "20014,20011",
+                               "-arch=sm_100a", "-diag-suppress", "20014,20011",
                                "-o", out, os.path.join(HOST, name + ".cu")])
         libs[name] = ctypes.CDLL(out)
     P, I = ctypes.c_void_p, ctypes.c_int

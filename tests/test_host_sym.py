@@ -30,6 +30,8 @@ def lib():
     for s in ("d", "f"):
         f = getattr(so, "host_sym_" + s)
         f.restype, f.argtypes = ctypes.c_long, [I, I, I, P, I, I, I, I, P, P, P, P, I, P, I]
+        f = getattr(so, "host_warp_" + s)
+        f.restype, f.argtypes = ctypes.c_long, [P, I, I, P, P, P]
     return so
 
 
@@ -88,3 +90,42 @@ def test_cluster_touches_only_running_ctas(lib, dtype, form, n, high_first):
     a = a0.astype(F64)
     assert np.linalg.norm(Q @ tridiagonal(d, e) @ Q.T - a) <= 8 * n * eps * np.linalg.norm(a)
     assert np.linalg.norm(Q.T @ Q - np.eye(n)) <= 8 * n * eps * n ** 0.5
+
+
+def reduce_warp(lib, a0):
+    n, dt = a0.shape[0], a0.dtype
+    A, d, e = a0.copy(), np.full(n, np.nan, dt), np.full(n, np.nan, dt)
+    f = lib.host_warp_d if dt == F64 else lib.host_warp_f
+    assert f(_p(A), n, n, None, _p(d), _p(e)) == 0
+    return d, e, A.T.astype(F64)
+
+
+@pytest.mark.parametrize("small_first", [False, True])
+@pytest.mark.parametrize("dtype,big,small", [
+    (F32, 1e10, 1e-5), (F32, 1e10, 1e-10), (F32, 1e10, 1e-12), (F32, 1e8, 1e-13), (F32, 1e16, 1e-14), (F32, 1, 1e-18),
+    (F64, 1e75, 1e-75), (F64, 1e100, 1e-60), (F64, 1e90, 1e-80), (F64, 1e145, 1e-140), (F64, 1, 1e-150)])
+@pytest.mark.parametrize("form,n", [("warp", 32), ("small", 50), ("cluster", 70)])
+def test_graded_blocks(lib, form, n, dtype, big, small, small_first):
+    """Block-diagonal matrices whose blocks differ by up to nearly the range
+    of the type: each block is reduced as if it were alone, A_b = Q_b T_b
+    Q_b^T to rounding of its own norm.  The reduction is backward stable block
+    by block because no reflector of one block has an entry in another."""
+    k = n // 2
+    lo, hi = (small, big) if small_first else (big, small)
+    a0 = np.zeros((n, n))
+    a0[:k, :k] = lo * uniform(k, F64, 1)
+    a0[k:, k:] = hi * uniform(n - k, F64, 2)
+    a0 = a0.astype(dtype)
+    if form == "warp":
+        d, e, Q = reduce_warp(lib, a0)
+    else:
+        f = {"small": {F64: (1, 2, 1), F32: (2, 1, 1)}, "cluster": {F64: (8, 2, 2), F32: (8, 4, 2)}}[form][dtype]
+        _, d, e, Q = reduce(lib, f, a0)
+    assert np.isfinite(d).all() and np.isfinite(e).all() and np.isfinite(Q).all()
+    eps = np.finfo(dtype).eps
+    T, a = tridiagonal(d, e), a0.astype(F64)
+    assert np.linalg.norm(Q.T @ Q - np.eye(n)) <= 8 * n * eps * n ** 0.5
+    for b in (slice(0, k), slice(k, n)):
+        s = np.abs(a[b, b]).max()
+        R = Q[b, b] @ (T[b, b] / s) @ Q[b, b].T - a[b, b] / s
+        assert np.linalg.norm(R) <= 8 * n * eps * np.linalg.norm(a[b, b] / s)
