@@ -76,6 +76,8 @@ cudaError_t dev_props(DevProps &out)
   return cudaSuccess;
 }
 
+constexpr size_t kSmemOptin = 227 * 1024;  // shared memory a block can have on sm_100
+
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Tuned options (eigen_GPU_batch_tune_set): per device, per (element size,
@@ -313,16 +315,32 @@ cudaError_t buffer_size(long L, int nm, int n, int m, size_t *lwork, const eigen
   return cudaSuccess;
 }
 
+// Static shared memory of a kernel, a property of the build; asked for once,
+// since asking costs microseconds.
+size_t static_smem(const void *kern)
+{
+  static std::map<const void *, size_t> known;
+  std::lock_guard<std::mutex> lk(g_mu);
+  auto it = known.find(kern);
+  if (it != known.end()) return it->second;
+  cudaFuncAttributes at;
+  if (cudaFuncGetAttributes(&at, kern) != cudaSuccess) {
+    cudaGetLastError();
+    return kSmemOptin;  // no dynamic shared memory beyond the default
+  }
+  return known[kern] = at.sharedSizeBytes;
+}
+
 // Admits a launch of kern with that much dynamic shared memory.  The limit set
-// is the same for every size (227 KB less the static shared memory of any
-// kernel here), so that of two threads whose calls launch one kernel at
-// different orders neither lowers the other's limit before its launch.  (A
-// constant of sm_100: asking the device costs 3 us a call.)
+// depends on the kernel alone: all that its static shared memory leaves.  So
+// of two threads whose calls launch one kernel at different orders neither
+// lowers the other's limit before its launch.
 template <class K> cudaError_t set_smem(K kern, size_t bytes)
 {
-  constexpr size_t fixed = 2 * 1024, all = 227 * 1024 - fixed;
-  if (bytes <= 48 * 1024 - fixed) return cudaSuccess;
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(bytes, all));
+  const size_t fixed = static_smem(reinterpret_cast<const void *>(kern));
+  if (bytes + fixed <= 48 * 1024) return cudaSuccess;
+  if (bytes + fixed > kSmemOptin) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemOptin - fixed));
 }
 
 // FP32 phase 1 in registers for 32 < n <= 64 (2 x 2 blocks of 32 x 32).  In

@@ -38,9 +38,12 @@ def test_tiles(dtype, n, nm, L):
         assert torch.equal(got, got.mT) and torch.isnan(z[:, :, n:]).all()
 
 
-def test_threads_of_different_orders():
+@pytest.mark.parametrize("orders", [(200, 250), (227, 200), (380, 300)])
+def test_threads_of_different_orders(orders):
     """Two host threads that launch the same kernels at different orders, each
-    on its own stream: every call succeeds and gives the bits of a lone one."""
+    on its own stream: every call succeeds and gives the bits of a lone one.
+    One kernel in each phase, other sizes of shared memory; 227 and 380 take all
+    but 2 KB of what a block can have."""
     import threading
     import eigeng_b200 as E
     out, errors = {}, []
@@ -63,7 +66,6 @@ def test_threads_of_different_orders():
         except Exception as e:  # noqa: BLE001
             errors.append((n, repr(e)))
 
-    orders = (200, 250)  # one kernel in each phase, other sizes of shared memory
     for n in orders:
         work(n, 1)
     threads = [threading.Thread(target=work, args=(n, 150)) for n in orders]
