@@ -265,35 +265,35 @@ __global__ void __launch_bounds__(32 * SPLIT, 1024 / (32 * SPLIT)) k1_cl(const K
                                reinterpret_cast<T *>(smem_raw));
 }
 
-template <class T, int NW, int RS, int CN, bool SCALED>
+template <class T, int NW, int RS, int CN, bool SCALED, bool ORD>
 __device__ __forceinline__ bool k1_sym_run(const KP<T> &p, const long k, const int m, const int stop,
                                            unsigned char *smem)
 {
   unsigned char *v = p.vw + (size_t)k * p.vstride;
-  return tridiag_sym<T, NW, RS, CN, SCALED>(
+  return tridiag_sym<T, NW, RS, CN, SCALED, ORD>(
       mat_ptr(p, k), p.nm, m, stop, m == p.n, p.ap && m == p.n ? p.ap + (size_t)k * packed_size(p.n) : nullptr,
       p.d + k * p.n, p.e + k * p.n, reinterpret_cast<T *>(v + fq_off_v(p.n)), fq_ldv(p.n),
       reinterpret_cast<double *>(v), reinterpret_cast<T *>(smem));
 }
-template <class T, int NW, int RS, int CN>
+template <class T, int NW, int RS, int CN, bool ORD>
 __device__ __noinline__ void k1_sym_again(const KP<T> &p, const long k, const int m, const int stop,
                                           unsigned char *smem)
 {
-  k1_sym_run<T, NW, RS, CN, true>(p, k, m, stop, smem);
+  k1_sym_run<T, NW, RS, CN, true, ORD>(p, k, m, stop, smem);
 }
 // Reduction of k1_sym<T, NW, RS, CN>: NW warps, RS blocks of a warp in
 // registers, CN CTAs per matrix (see eigb_tridiag_sym.cuh and sym_cfg), of the
 // leading m x m block down to order `stop`.
-template <class T, int NW, int RS, int CN, int MB>
+template <class T, int NW, int RS, int CN, int MB, bool ORD = sym_ord<T>(NW, CN)>
 __global__ void __launch_bounds__(32 * NW, MB) k1_sym(const __grid_constant__ KP<T> p, const int m, const int stop)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const long k = blockIdx.x / CN;
   // The second run is a call in FP64 and inline in FP32: the other way round
   // FP64 n=512 L=256 takes 1.8 % longer (spills), FP32 n=128 L=4096 1.6 %.
-  if (k1_sym_run<T, NW, RS, CN, false>(p, k, m, stop, smem_raw)) {
-    if (sizeof(T) == 4) k1_sym_run<T, NW, RS, CN, true>(p, k, m, stop, smem_raw);
-    else k1_sym_again<T, NW, RS, CN>(p, k, m, stop, smem_raw);
+  if (k1_sym_run<T, NW, RS, CN, false, ORD>(p, k, m, stop, smem_raw)) {
+    if (sizeof(T) == 4) k1_sym_run<T, NW, RS, CN, true, ORD>(p, k, m, stop, smem_raw);
+    else k1_sym_again<T, NW, RS, CN, ORD>(p, k, m, stop, smem_raw);
   }
 }
 

@@ -193,6 +193,47 @@ template <class T> __device__ __forceinline__ T warp_max(T x)
   return x;
 }
 
+// Sums of the one-CTA forms in an order that does not depend on the form (NW,
+// RS), so that batches of any size, whose launches hand over at other orders
+// (sym_next), give the same bits: |v|^2 by row blocks of 32, v.Av by blocks l %
+// 8, those of a group from the last to the first.  The form of a cluster
+// is fixed by the order instead, the two-warp forms of FP32 are in no chain, and
+// orders up to 64 have but one form (ORD false).  Costs up to 1.6 % of a solve
+// (FP64 n=128 L=4096 8.96 -> 9.11 ms, n=256 L=2048 32.48 -> 32.57); hand-overs at
+// fixed orders instead would cost small batches 2 to 6 %, none at all large ones
+// 2 to 4 %.
+template <class T> __host__ __device__ constexpr bool sym_ord(int nw, int cn)
+{
+  return cn == 1 && (sizeof(T) == 8 || nw > 2);
+}
+// Two and four sums over a warp at once, with the additions of warp_sum: the
+// one that sym_slot2 or sym_slot4 names.
+template <class T> __device__ __forceinline__ T sym_half(const T a, const T b, const bool hi, const int o)
+{
+  T mine = a, other = b;
+  if (hi) mine = b;
+  if (hi) other = a;
+  return mine + __shfl_xor_sync(0xffffffffu, other, o);
+}
+template <class T> __device__ __forceinline__ T sym_sum8(T s)
+{
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+__device__ __forceinline__ int sym_slot2(const int lane) { return lane >> 4; }
+template <class T> __device__ __forceinline__ T sym_sum2(const T a, const T b, const int lane)
+{
+  const T s = sym_half(a, b, lane & 16, 16);
+  return sym_sum8(s + __shfl_xor_sync(0xffffffffu, s, 8));
+}
+__device__ __forceinline__ int sym_slot4(const int lane) { return lane >> 3; }
+template <class T> __device__ __forceinline__ T sym_sum4(const T a, const T b, const T c, const T d, const int lane)
+{
+  const T x = sym_half(a, c, lane & 16, 16), y = sym_half(b, d, lane & 16, 16);
+  return sym_sum8(sym_half(x, y, lane & 8, 8));
+}
+
 // One step i (i = n-1 .. 1) removes column i with the reflector u whose raw
 // entries v are the rows < i of that column: u = v - anorm e_{i-1}, so
 //   A u = A v - anorm A e_{i-1},   u.A u = v.Av - 2 anorm (A v)_{i-1} + anorm^2 A_{i-1,i-1},
@@ -210,15 +251,19 @@ template <class T> __device__ __forceinline__ T warp_max(T x)
 //   barrier  (cluster)
 //
 // Reduces the leading n x n block of A down to order `stop` (0: to the end),
-// where it leaves the updated leading block in A's upper triangle for a call
+// where it leaves the updated leading block in A's blocks (R <= C) for a call
 // with fewer warps or CTAs; `first` is the call on the whole matrix.  Returns
 // true if it has to be run again with SCALED; A is as it was then.
-template <class T, int NW, int RS, int CN, bool SCALED>
+template <class T, int NW, int RS, int CN, bool SCALED, bool ORD = sym_ord<T>(NW, CN)>
 __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, const int stop, const bool first,
                                             const T *Ap, T *d_out, T *e_out, T *V, const int ldv, double *beta_out,
                                             T *sm)
 {
   constexpr int NT = 32 * NW;
+  // a warp's groups of blocks, and the posted sums that can differ from 0
+  constexpr int NG = !ORD ? 1 : (NW < 2 ? 4 : 8 / NW);
+  constexpr int NSG = !ORD ? NW : (2 * NW < (sizeof(T) == 8 ? 8 : 12) ? 2 * NW : (sizeof(T) == 8 ? 8 : 12));
+  constexpr int NDT = !ORD ? NW : (NW < 2 ? 4 : 8);
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int rank = CN > 1 ? (int)(blockIdx.x % CN) : 0;
   const int nbk = sym_nbk(n), nr = 32 * nbk, nblk = sym_nblk(n), nl = sym_local(n, CN);
@@ -237,7 +282,9 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
 
   const int lr = lane & 3, lc = lane >> 2, xj = lane >> 3, xh = (lane >> 1) & 1;
   auto elem = [&](int r, int c) -> T {  // element (r, c) of the input, 0 outside
-    const int a = min(r, c), b = max(r, c);
+    // the blocks on the diagonal are kept in full, their halves rounded apart, and handed over so
+    const int a = first ? min(r, c) : r, b = first ? max(r, c) : c;
+    if (!first && r >= n) return T(0);
     if (b >= n) return T(0);
     return Ap ? Ap[a + (size_t)b * (b + 1) / 2] : A[a + (size_t)b * nm];
   };
@@ -339,7 +386,7 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
       } else {
         T a1 = T(0);
 #pragma unroll
-        for (int q = 0; q < NW; q += 2) {
+        for (int q = 0; q < NDT; q += 2) {
           T x0, x1;
           sld2(dotp + q, x0, x1);
           dsum += x0;
@@ -360,7 +407,7 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
     const T uau = fma(anorm * anorm, ci, fma(T(-2) * anorm, yi, dsum));
     const T alpha = T(0.5) * beta * (beta * uau);
     const T wi = fma(alpha, ul, pi);
-    T sig = T(0);
+    T sig = T(0), sig1 = T(0);  // of the warp's first row block, and its second
     for (int r = t; r < nr; r += NT) {
       T *xr = uwv + 96 * (r >> 5) + (r & 31);
       T u = T(0), w = T(0), v = T(0);
@@ -400,7 +447,9 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
       xr[0] = u;
       xr[32] = w;
       xr[64] = v;
-      sig = fma(v, v, sig);
+      const bool second = ORD && r != t;
+      sig1 = second ? v * v : sig1;
+      sig = second ? sig : fma(v, v, sig);
     }
     if (i == 0) break;
     if (i < stop) {  // i = stop - 1: the pending update alone, and the block goes out
@@ -417,7 +466,7 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
         for (int x = 0; x < 32; x++) {
           const int r = 2 * lr + 8 * ((x >> 3) ^ xj) + ((x >> 2) & 1), c = 2 * lc + 16 * (((x >> 1) & 1) ^ xh) + (x & 1);
           const T v = fma(xR[32 + r], xC[c], fma(xR[r], xC[32 + c], get(x)));
-          if (32 * R + r <= 32 * C + c) A[32 * R + r + (size_t)(32 * C + c) * nm] = v * back;
+          A[32 * R + r + (size_t)(32 * C + c) * nm] = v * back;
         }
       };
       const int nout = (stop / 32) * (stop / 32 + 1) / 2;
@@ -430,12 +479,17 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
         if ((s * NW + warp) * CN + rank < nout) out(s * NW + warp, [&](const int x) { return S[s][x]; });
       return false;
     }
-    sig = warp_sum(sig);
-    if (lane == 0) sg[warp] = sig;
+    if (!ORD) {
+      sig = warp_sum(sig);
+      if (lane == 0) sg[warp] = sig;
+    } else {
+      sig = sym_sum2(sig, sig1, lane);
+      if ((lane & 15) == 0) sg[warp + NW * sym_slot2(lane)] = sig;
+    }
     __syncthreads();
     if constexpr (SCALED) {
       T s = T(0), eb = T(1);
-      for (int q = 0; q < NW; q++) s += sg[q];
+      for (int q = 0; q < NSG; q++) s += sg[q];
       if (s < sym_tiny<T>()) {
         T mv = T(0), up;
         for (int r = t; r < nr; r += NT) mv = fmax_t(mv, fabs_t(uwv[96 * (r >> 5) + 64 + (r & 31)]));
@@ -444,14 +498,22 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
         __syncthreads();
         for (int q = 0; q < NW; q++) mv = fmax_t(mv, dotp[q]);
         sym_pow2(mv, 0, up, eb);
-        s = T(0);
+        sig = sig1 = T(0);
         for (int r = t; r < nr; r += NT) {
-          T *v = uwv + 96 * (r >> 5) + 64 + (r & 31);
-          *v *= up;
-          s = fma(*v, *v, s);
+          T *x = uwv + 96 * (r >> 5) + 64 + (r & 31);
+          const T v = *x * up;
+          *x = v;
+          const bool second = ORD && r != t;
+          sig1 = second ? v * v : sig1;
+          sig = second ? sig : fma(v, v, sig);
         }
-        s = warp_sum(s);
-        if (lane == 0) sg[warp] = s;
+        if (!ORD) {
+          sig = warp_sum(sig);
+          if (lane == 0) sg[warp] = sig;
+        } else {
+          sig = sym_sum2(sig, sig1, lane);
+          if ((lane & 15) == 0) sg[warp + NW * sym_slot2(lane)] = sig;
+        }
       }
       if (t == 0) sc[4] = eb;
       __syncthreads();
@@ -461,7 +523,7 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
     if (warp == NW - 1) {
       T s0 = T(0), s1 = T(0);
 #pragma unroll
-      for (int q = 0; q < NW; q += 2) {
+      for (int q = 0; q < NSG; q += 2) {
         T x0, x1;
         sld2(sg + q, x0, x1);
         s0 += x0;
@@ -491,7 +553,9 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
     // ---- pass over the blocks ----
     const int ca = (i - 1) >> 5;  // last active block column, which holds column i-1
     const int par = (i - 1) & 1;
-    T dot = T(0);
+    T dot[NG];
+#pragma unroll
+    for (int a = 0; a < NG; a++) dot[a] = T(0);
     const int myr = 2 * lr + 8 * xj + ((lane >> 2) & 1);
     const int myc = 2 * lc + 16 * xh + (lane & 1);
     auto put_col = [&](const int R) {
@@ -505,9 +569,10 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
         }
       };
     };
-    for (int l = RS * NW + warp; l < nl; l += NW) {  // blocks in shared memory
+    // blocks in shared memory, from the last active one
+    const int nact1 = ((ca + 1) * (ca + 2) / 2 - rank + CN - 1) / CN - 1 - warp;  // local blocks active, less 1 + warp
+    for (int l = warp + (nact1 & ~(NW - 1)); l >= RS * NW; l -= NW) {
       const int g = l * CN + rank;
-      if (g >= (ca + 1) * (ca + 2) / 2) break;
       int C = (int)((sqrtf(8.0f * (float)g + 1.0f) - 1.0f) * 0.5f);
       if ((C + 1) * (C + 2) / 2 <= g) C++;
       if (C * (C + 1) / 2 > g) C--;
@@ -521,10 +586,15 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
           C == ca ? ((i - 1) & 31) : -1, put_col(R), rsum, csum);
       prow[l * 32 + myr] = rsum;
       pcol[l * 32 + myc] = csum;
-      dot = fma(rsum * (R == C ? T(1) : T(2)), uwv[96 * R + 64 + myr], dot);
+      const T z = rsum * (R == C ? T(1) : T(2)), vr = uwv[96 * R + 64 + myr];
+#pragma unroll
+      for (int a = 0; a < NG; a++) {
+        const T x = fma(z, vr, dot[a]);
+        dot[a] = NG == 1 || (l & 7) / NW == a ? x : dot[a];
+      }
     }
 #pragma unroll
-    for (int s = 0; s < RS; s++) {
+    for (int s = RS - 1; s >= 0; s--) {
       if (bC[s] <= ca) {
         const int R = bR[s], C = bC[s], l = s * NW + warp;
         T rsum, csum;
@@ -541,11 +611,19 @@ __device__ __forceinline__ bool tridiag_sym(T *A, const int nm, const int n, con
             C == ca ? ((i - 1) & 31) : -1, put_col(R), rsum, csum);
         prow[l * 32 + myr] = rsum;
         pcol[l * 32 + myc] = csum;
-        dot = fma(rsum * (R == C ? T(1) : T(2)), uwv[96 * R + 64 + myr], dot);
+        dot[s % NG] = fma(rsum * (R == C ? T(1) : T(2)), uwv[96 * R + 64 + myr], dot[s % NG]);
       }
     }
-    dot = warp_sum(dot);
-    if (lane == 0) dotp[warp] = dot;
+    if constexpr (NG == 4) {
+      const T x = sym_sum4(dot[0], dot[1], dot[2], dot[3], lane);
+      if ((lane & 7) == 0) dotp[warp + NW * sym_slot4(lane)] = x;
+    } else if constexpr (NG == 2) {
+      const T x = sym_sum2(dot[0], dot[1], lane);
+      if ((lane & 15) == 0) dotp[warp + NW * sym_slot2(lane)] = x;
+    } else {
+      const T x = warp_sum(dot[0]);
+      if (lane == 0) dotp[warp] = x;
+    }
     __syncthreads();
 
     if (CN > 1) {

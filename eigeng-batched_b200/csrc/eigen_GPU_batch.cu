@@ -25,6 +25,7 @@
 #include "eigb_refine.cuh"
 #include "eigb_learned.cuh"
 #include "eigb_queue.cuh"
+#include "eigb_sym_cfg.cuh"
 #include "../../include/eigen_GPU_learned.h"
 #include "../../include/eigen_GPU_batch.h"
 
@@ -351,50 +352,12 @@ template <class K> cudaError_t set_smem(K kern, size_t bytes)
 template <class T> bool reg_form(int n) { return sizeof(T) == 4 && n > 32 && n <= 64; }
 template <class T> size_t k1r_smem_bytes(int n) { return sizeof(T) * reg_smem_elems<2>(n); }
 
-// k1_sym: warps, blocks per warp in registers and CTAs per matrix
-struct SymCfg {
-  int nw, rs, cn, mb;  // mb: CTAs an SM the registers are bounded for
-};
-// Measured on B200 (the reduction alone, ms).  Where several matrices fit an
-// SM, small CTAs with few blocks in registers win, their step chains hiding
-// one another: FP64 n=64 L=20000 one warp x 2 blocks 2.85, two x 1 3.26, four
-// x 1 4.43; n=96 L=8000 two x 1, six CTAs 3.07, four x 1 3.40; n=128 L=4096 4 warps x 1 block, three CTAs 3.04, x 2
-// blocks, two CTAs 3.48, 8 x 2, one CTA 5.62; n=160 L=3000 4.65 / 4.05 /
-// 5.69.  From n = 161 on 4 warps no longer have two CTAs an SM (n=192 L=2048
-// 6.58 against 5.20 with 8).  Above 256 the fewest CTAs that hold the
-// triangle: n=512 L=256 4 CTAs 13.4, 8 CTAs 28.8; n=384 L=512 15.3 / 36.8;
-// n=736 L=64 8 CTAs 15.6, 16 CTAs 29.2.  FP32: n=96 L=8000 2 x 1,
-// eight CTAs 1.67, 4 x 1 2.07; n=128 L=4096 2 x 2 1.66, 4 x 1 1.76; n=160 L=3000 4 x 1 2.14, 8 x 1
-// 2.80; n=224 L=2048 4.33 / 3.53; n=256 8 x 1 7.06, 4 x 4 5.04, 8 x 4 6.28;
-// n=288 L=1024 4 x 4 5.79, 8 x 4 4.03; n=1000 L=32 8 CTAs 14.2, 16 21.1.
-template <class T> SymCfg sym_cfg(int n)
-{
-  if (sizeof(T) == 8) {
-    if (n <= 64) return {1, 2, 1, 8};
-    if (n <= 96) return {2, 1, 1, 6};
-    if (n <= 128) return {4, 1, 1, 3};
-    if (n <= 160) return {4, 2, 1, 2};
-    if (n <= 256) return {8, 2, 1, 1};
-    if (n <= 352) return {8, 2, 2, 1};
-    if (n <= 512) return {8, 2, 4, 1};
-    if (n <= 736) return {8, 2, 8, 1};
-    return {8, 2, 16, 1};
-  }
-  if (n <= 96) return {2, 1, 1, 8};
-  if (n <= 128) return {2, 2, 1, 6};
-  if (n <= 160) return {4, 1, 1, 4};
-  if (n <= 224) return {8, 1, 1, 2};
-  if (n <= 256) return {4, 4, 1, 2};
-  if (n <= 384) return {8, 4, 1, 1};
-  if (n <= 512) return {8, 4, 2, 1};
-  if (n <= 736) return {8, 4, 4, 1};
-  return {8, 4, 8, 1};
-}
 template <class T> using SymKernel = void (*)(const KP<T>, const int, const int);
-template <class T> SymKernel<T> sym_kernel(const SymCfg &c)
+// `own`: the solve's order is the launch's (ORD of tridiag_sym does not matter up to 64)
+template <class T> SymKernel<T> sym_kernel(const SymCfg &c, const bool own)
 {
   if constexpr (sizeof(T) == 8) {
-    if (c.nw == 1) return k1_sym<T, 1, 2, 1, 8>;
+    if (c.nw == 1) return own ? k1_sym<T, 1, 2, 1, 8, false> : k1_sym<T, 1, 2, 1, 8>;
     if (c.nw == 2) return k1_sym<T, 2, 1, 1, 6>;
     if (c.nw == 4) return c.rs == 1 ? k1_sym<T, 4, 1, 1, 3> : k1_sym<T, 4, 2, 1, 2>;
     switch (c.cn) {
@@ -420,24 +383,6 @@ template <class T> size_t sym_smem(int n, const SymCfg &c)
 {
   return sizeof(T) * sym_smem_elems(n, c.nw, c.rs, c.cn);
 }
-// Order at which a reduction that began at n hands the leading block over to a
-// launch with fewer CTAs or warps (0: none).  A matrix keeps its SMs to the
-// last step otherwise, and the last steps have little to do; where the batch
-// takes more than one wave of CTAs, another launch packs the small blocks
-// closer.  Measured on B200 (the reduction, ms, without / with): FP64 n=72
-// L=8000 1.96 / 1.78, n=96 L=8000 3.09 / 2.89, n=128 L=4096 3.05 / 2.81, n=160
-// L=3000 4.20 / 3.84, n=256 L=2048 9.68 / 8.39, n=512 L=256 14.0 / 10.3, n=1000
-// L=32 26.9 / 18.2; FP32 n=201 L=1000 1.57 / 1.37, n=512 L=256 6.80 / 5.30,
-// n=1000 L=32 14.1 / 9.3.  In a single wave it costs: FP64 n=512 L=32 1.76 /
-// 2.12.
-template <class T> int sym_next(int n, long cnt, const SymCfg &c, int sms)
-{
-  if (cnt * c.cn <= (long)sms * c.mb) return 0;
-  const int at64[] = {736, 512, 352, 256, 128, 64, 0}, at32[] = {736, 512, 384, 160, 0};
-  const int *at = sizeof(T) == 8 ? at64 : at32;
-  while (*at >= n) at++;
-  return *at;
-}
 template <class T> cudaLaunchConfig_t sym_launch(int n, const SymCfg &c, long cnt, cudaStream_t st,
                                                  cudaLaunchAttribute *at)
 {
@@ -456,11 +401,11 @@ template <class T> cudaLaunchConfig_t sym_launch(int n, const SymCfg &c, long cn
 }
 // sets the kernel's attributes and says whether the device can run it (a
 // cluster of 16 needs a GPU processing cluster with that many SMs)
-template <class T> bool sym_usable(int n, const SymCfg &c, const DevProps &dp)
+template <class T> bool sym_usable(int n, const SymCfg &c, const DevProps &dp, const bool own = true)
 {
   const size_t smem = sym_smem<T>(n, c);
   if (n <= 32 || reg_form<T>(n) || smem > (size_t)dp.smem_optin) return false;
-  SymKernel<T> kern = sym_kernel<T>(c);
+  SymKernel<T> kern = sym_kernel<T>(c, own);
   if (set_smem(kern, smem) != cudaSuccess) return false;
   if (c.cn == 1) return true;
   if (c.cn > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
@@ -505,11 +450,11 @@ cudaError_t launch_sym(const KP<T> &p, const DevProps &dp, const FormQ<T> &f, lo
 {
   for (int m = p.n; m > 0;) {
     const SymCfg c = sym_cfg<T>(m);
-    int stop = sym_next<T>(m, cnt, c, dp.sms);
-    if (stop && !sym_usable<T>(stop, sym_cfg<T>(stop), dp)) stop = 0;  // also sets the next kernel's attributes
+    int stop = sym_next<T>(m, cnt, dp.sms);
+    if (stop && !sym_usable<T>(stop, sym_cfg<T>(stop), dp, false)) stop = 0;  // also sets the next kernel's attributes
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = sym_launch<T>(m, c, cnt, st, at);
-    const cudaError_t err = cudaLaunchKernelEx(&cfg, sym_kernel<T>(c), p, m, stop);
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, sym_kernel<T>(c, m == p.n), p, m, stop);
     if (err != cudaSuccess) return err;
     m = stop;
   }

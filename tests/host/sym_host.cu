@@ -2,6 +2,7 @@
 // eigb_tridiag_warp.cuh), run by tests/host/simt.hpp.
 #include "simt.hpp"
 
+#include "../../eigeng-batched_b200/csrc/eigb_sym_cfg.cuh"
 #include "../../eigeng-batched_b200/csrc/eigb_tridiag_sym.cuh"
 #include "../../eigeng-batched_b200/csrc/eigb_tridiag_warp.cuh"
 
@@ -57,7 +58,27 @@ template <class T> static long warp(T *A, int nm, int n, const T *Ap, T *d, T *e
   });
 }
 
+// The launches of the reduction of order n for cnt matrices on 148 SMs, as the
+// library chooses them: four ints each (order, warps, blocks in registers,
+// CTAs); returns their number.
+template <class T> static int chain(int n, long cnt, int *out)
+{
+  int k = 0;
+  for (int m = n; m > 0; m = eigb::sym_next<T>(m, cnt, 148), k++) {
+    const eigb::SymCfg c = eigb::sym_cfg<T>(m);
+    out[4 * k] = m;
+    out[4 * k + 1] = c.nw;
+    out[4 * k + 2] = c.rs;
+    out[4 * k + 3] = c.cn;
+  }
+  return k;
+}
+
 extern "C" {
+int host_sym_chain(int esize, int n, long cnt, int *out)
+{
+  return esize == 8 ? chain<double>(n, cnt, out) : chain<float>(n, cnt, out);
+}
 long host_warp_d(double *A, int nm, int n, const double *Ap, double *d, double *e) { return warp(A, nm, n, Ap, d, e); }
 long host_warp_f(float *A, int nm, int n, const float *Ap, float *d, float *e) { return warp(A, nm, n, Ap, d, e); }
 long host_sym_d(int nw, int rs, int cn, double *A, int nm, int m, int stop, int first, const double *Ap, double *d,

@@ -93,8 +93,7 @@ def test_packed_input_and_special_matrices(oracle_mod, dtype, n):
 @pytest.mark.parametrize("dtype,n,L", [("f64", 65, 900), ("f64", 96, 900), ("f64", 128, 460), ("f64", 129, 300),
                                        ("f64", 353, 60), ("f32", 161, 310), ("f32", 385, 80)])
 def test_more_than_a_wave_of_matrices(dtype, n, L):
-    """Batches of more than one wave of CTAs hand their leading blocks over to
-    launches of smaller CTAs; every matrix still comes back as Q T Q^T."""
+    """Batches of more than one wave of CTAs; every matrix comes back as Q T Q^T."""
     import eigeng_b200 as E
     dt = torch.float64 if dtype == "f64" else torch.float32
     g = torch.Generator(device="cuda")
@@ -109,3 +108,36 @@ def test_more_than_a_wave_of_matrices(dtype, n, L):
     res = torch.linalg.matrix_norm(Qt.mT @ T @ Qt - A) / torch.linalg.matrix_norm(A)
     orth = torch.linalg.matrix_norm(Qt @ Qt.mT - torch.eye(n, dtype=torch.float64, device="cuda")) / n ** 0.5
     assert res.max().item() <= 8 * n * eps and orth.max().item() <= 8 * n * eps, (res.max(), orth.max())
+
+
+@pytest.mark.parametrize("dtype,n,L", [("f64", 72, 900), ("f64", 128, 460), ("f64", 200, 160), ("f64", 400, 40),
+                                       ("f32", 200, 310), ("f32", 600, 40)])
+def test_parts_of_a_batch_give_the_same_bits(dtype, n, L):
+    """A batch of more than one wave of CTAs, and parts of it that are less: in
+    internal chunks, through the stages in two parts, packed, and as a mixed
+    batch, every matrix has the eigenpairs of the one call, bit for bit."""
+    import eigeng_b200 as E
+    dt = torch.float64 if dtype == "f64" else torch.float32
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    x = (torch.rand((L, n, n), generator=g, device="cuda", dtype=torch.float64) * 2 - 1).to(dt)
+    a0 = x.tril() + x.tril(-1).mT
+    a = a0.clone()
+    w, info = E.solve(a, n)
+    b = a0.clone()
+    wb, _ = E.solve(b, n, chunk=L // 3)
+    s = a0.clone()
+    ws, infos = torch.empty_like(w), torch.empty_like(info)
+    wk = E.workspace(L, n, n, dt, chunk=L)
+    for first, count in ((0, L // 2), (L // 2, L - L // 2)):
+        assert E.stage(s, ws, wk, n, E.STAGE_ALL, first, count, info=infos) == 0
+    zp, wp, _ = E.solve_packed(E.pack_upper(a0[:7], n), n)
+    k = 5
+    u = torch.cat([a0[:k].reshape(-1), a0[0, :40, :40].reshape(-1)])
+    wu, _ = E.solve_uneven(u, [n] * k + [40])
+    torch.cuda.synchronize()
+    assert (info == 0).all() and (infos == 0).all()
+    assert torch.equal(b, a) and torch.equal(wb, w)
+    assert torch.equal(s, a) and torch.equal(ws, w)
+    assert torch.equal(zp, a[:7]) and torch.equal(wp, w[:7])
+    assert torch.equal(u[:k * n * n].view(k, n, n), a[:k]) and torch.equal(wu[:k * n].view(k, n), w[:k])

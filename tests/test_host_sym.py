@@ -129,3 +129,75 @@ def test_graded_blocks(lib, form, n, dtype, big, small, small_first):
         s = np.abs(a[b, b]).max()
         R = Q[b, b] @ (T[b, b] / s) @ Q[b, b].T - a[b, b] / s
         assert np.linalg.norm(R) <= 8 * n * eps * np.linalg.norm(a[b, b] / s)
+
+
+def chain(lib, dtype, n, cnt):
+    """[(order, form)]: the launches that the library's rule gives cnt matrices of order n."""
+    out = np.zeros(64, np.int32)
+    k = lib.host_sym_chain(np.dtype(dtype).itemsize, n, ctypes.c_long(cnt), _p(out))
+    return [(int(x[0]), tuple(int(y) for y in x[1:])) for x in out.reshape(-1, 4)[:k]]
+
+
+def run_chain(lib, launches, a0):
+    n, dt = a0.shape[0], a0.dtype
+    A, V = a0.copy(), np.full((n, (n + 7) & ~7), np.nan, dt)
+    d, e, beta = np.full(n, np.nan, dt), np.full(n, np.nan, dt), np.full(n, np.nan)
+    for q, (m, form) in enumerate(launches):
+        stop = launches[q + 1][0] if q + 1 < len(launches) else 0
+        assert launch(lib, form, A, m, stop, int(q == 0), d, e, V, beta) == 0
+    return d, e, reflectors(V, beta)
+
+
+MANY = [(F64, 72, [72, 64]), (F64, 96, [96, 64]), (F64, 128, [128, 64]), (F64, 130, [130, 128, 64]),
+        (F64, 161, [161, 128, 64]), (F64, 256, [256, 128, 64]), (F32, 170, [170, 160]), (F32, 230, [230, 160]),
+        (F32, 290, [290, 160])]
+
+
+@pytest.mark.parametrize("dtype,n,orders", MANY)
+def test_small_and_large_batches_give_the_same_bits(lib, dtype, n, orders):
+    """A batch of more than one wave of CTAs hands its leading blocks over to
+    smaller ones, a single matrix does not: the same d, e and Q, bit for bit,
+    and A = Q T Q^T."""
+    many, one = chain(lib, dtype, n, 100000), chain(lib, dtype, n, 1)
+    assert [m for m, _ in many] == orders and [m for m, _ in one] == [n]
+    a0 = uniform(n, dtype, n)
+    d, e, Q = run_chain(lib, many, a0)
+    d1, e1, Q1 = run_chain(lib, one, a0)
+    assert np.array_equal(d, d1) and np.array_equal(e, e1) and np.array_equal(Q, Q1)
+    eps, a = np.finfo(dtype).eps, a0.astype(F64)
+    assert np.linalg.norm(Q @ tridiagonal(d, e) @ Q.T - a) <= 8 * n * eps * np.linalg.norm(a)
+    assert np.linalg.norm(Q.T @ Q - np.eye(n)) <= 8 * n * eps * n ** 0.5
+
+
+@pytest.mark.parametrize("dtype,n", [(F64, 130), (F64, 260), (F32, 170)])
+def test_graded_blocks_across_a_hand_over(lib, dtype, n):
+    """Blocks of very different magnitude, block by block as if alone, with the
+    border between them at another order than the hand-overs."""
+    launches = chain(lib, dtype, n, 100000)
+    assert len(launches) > 1
+    k = n // 2
+    a0 = uniform(n, dtype, n)
+    a0[:k, k:] = a0[k:, :k] = 0
+    a0[:k, :k] *= dtype(1e-20 if dtype == F32 else 1e-200)
+    d, e, Q = run_chain(lib, launches, a0)
+    T, eps, a = tridiagonal(d, e), np.finfo(dtype).eps, a0.astype(F64)
+    assert np.linalg.norm(Q.T @ Q - np.eye(n)) <= 8 * n * eps * n ** 0.5
+    for b in (slice(0, k), slice(k, n)):
+        s = np.abs(a[b, b]).max()
+        R = Q[b, b] @ (T[b, b] / s) @ Q[b, b].T - a[b, b] / s
+        assert np.linalg.norm(R) <= 8 * n * eps * np.linalg.norm(a[b, b] / s)
+
+
+def test_chain_of_every_order(lib):
+    """The launches shrink to the end; those of more than one CTA a matrix,
+    which sum in another order, are the same for every batch."""
+    for dtype in (F64, F32):
+        for n in range(33, 1025):
+            few, many = chain(lib, dtype, n, 1), chain(lib, dtype, n, 100000)
+            for c in (few, many):
+                assert c[0][0] == n and all(x[0] > y[0] for x, y in zip(c, c[1:]))
+            assert [x for x in few if x[1][2] > 1] == [x for x in many if x[1][2] > 1]
+    for n, few, many in ((1000, [736, 512, 256], [736, 512, 256, 128, 64]), (513, [512, 256], [512, 256, 128, 64]),
+                         (300, [256], [256, 128, 64])):
+        assert [m for m, _ in chain(lib, F64, n, 1)] == [n] + few
+        assert [m for m, _ in chain(lib, F64, n, 100000)] == [n] + many
