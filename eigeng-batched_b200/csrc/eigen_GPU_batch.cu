@@ -829,11 +829,9 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
   return cudaSuccess;
 }
 
-// Launch geometry of the reduction in its one-CTA-per-matrix form (or the
-// cluster form where the tuned options ask for it), for the first chunk of a
-// default solve; the counterpart of the reference's
-// eigen_GPU_batch_get_Launch_params (eigen_GPU_batch.hpp:23-102).  Above
-// n = 64 run() spreads a matrix otherwise (sym_cfg) where the device can.
+// Launch geometry of phase 1 (the matrix-parallel reduction) for the first
+// chunk of a default solve, as run() launches it; the counterpart of the
+// reference's eigen_GPU_batch_get_Launch_params (eigen_GPU_batch.hpp:23-102).
 template <class T>
 cudaError_t launch_params(long L, int n, int *grp, int *tb, int *gr, int *th, int *sh, int *l2)
 {
@@ -867,12 +865,17 @@ cudaError_t launch_params(long L, int n, int *grp, int *tb, int *gr, int *th, in
     *th = 32 * K1W_NW;
     *tb = (int)((lc + K1W_NW - 1) / K1W_NW);
     *sh = (int)(sizeof(T) * tw_smem_elems() * K1W_NW);
-  } else if (n <= 128) {  // the register form: NB x NB warps
-    const int nb = (n + 31) / 32;
-    *grp = *th = 32 * nb * nb;
+  } else if (reg_form<T>(n)) {  // k1_reg: 2 x 2 warps
+    *grp = *th = 32 * 4;
     *gr = 1;
     *tb = (int)lc;
-    *sh = (int)(sizeof(T) * (nb == 2 ? reg_smem_elems<2>(n) : (nb == 3 ? reg_smem_elems<3>(n) : reg_smem_elems<4>(n))));
+    *sh = (int)k1r_smem_bytes<T>(n);
+  } else if (const SymCfg c = sym_cfg<T>(n); sym_usable<T>(n, c, dp)) {  // k1_sym, its launch on the whole matrices
+    *th = 32 * c.nw;
+    *grp = c.cn * *th;
+    *gr = 1;
+    *tb = (int)(lc * c.cn);
+    *sh = (int)sym_smem<T>(n, c);
   } else {  // k1_cta
     *grp = *th = k1c_threads<T>(n);
     *gr = 1;

@@ -355,14 +355,13 @@ cudaError_t eigen_GPU_batch_symfunc_FP(const int L, const int nm, const int n, c
  * kernel) of a default solve of L matrices of order n on the current
  * device, for the first chunk of the batch; counterpart of the reference's
  * header-only eigen_GPU_batch_get_Launch_params (eigen_GPU_batch.hpp:23-102),
- * which include/eigen_GPU_batch.hpp forwards here.  The geometry is that of
- * the one-CTA-per-matrix form in full storage (what a caller who sizes by
- * threads per matrix wants); above n = 64 the solve itself spreads a matrix
- * over fewer threads or over a cluster.  grpSZ: threads that own
- * one matrix; numGR: matrices per thread block (1 also for the cluster
- * form, where a matrix spans a cluster of ceil(n/32) blocks and grpSZ
- * counts the cluster's threads); numTH: threads per block; numTB: thread
- * blocks of the launch; sizeSH: dynamic shared memory bytes per block;
+ * which include/eigen_GPU_batch.hpp forwards here.  grpSZ: threads that own
+ * one matrix; numGR: matrices per thread block (1 also where a matrix spans
+ * a cluster of blocks: FP64 n > 256, FP32 n > 384, and the tuned cluster
+ * form; grpSZ then counts the cluster's threads); numTH: threads per block;
+ * numTB: thread blocks of the launch that takes the whole matrices (the last
+ * steps of larger orders run in further launches of fewer threads); sizeSH:
+ * dynamic shared memory bytes per block;
  * sizeL2: the device's L2 bytes.  cudaErrorInvalidValue for L < 1, n < 1
  * or n > 1024.
  */

@@ -87,16 +87,14 @@ import pytest  # noqa: E402
 def test_launch_params_report_the_launched_geometry(tmp_path):
     """eigen_GPU_batch_get_Launch_params<T> reports phase 1 as run() launches
     it: one thread per matrix for n = 1, a warp per matrix (four per block)
-    for n <= 32, a CTA of 32*NB*NB threads (NB = ceil(n/32)) in the
-    register form for 32 < n <= 128, and the CTA form's
-    min(1024, ceil(n/32)*32*split) threads above (FP64 split 2 up to n =
-    240, 4 up to 256, 2 up to 512, then 1), one block per matrix; with the cluster form asked
-    for (tuned option reduce), ceil(n/32) blocks of 512 threads per
-    matrix."""
+    for n <= 32, above in FP64 one block of 1, 2, 4 or 8 warps per matrix up to
+    n = 64, 96, 160 and 256, then 2, 4, 8 and 16 blocks of 8 warps up to n =
+    352, 512, 736 and 1024; FP32 n = 64 the register form's 128 threads; with the
+    cluster form asked for (tuned option reduce), ceil(n/32) blocks of 512
+    threads per matrix."""
     import subprocess
     out = subprocess.check_output([_cpp_launch_params_program(str(tmp_path))], text=True)
     rows = {int(x.split()[0]): [int(v) for v in x.split()[1:]] for x in out.strip().splitlines()}
-    import math
     for n, (g, b, r, t, s, l) in rows.items():
         assert l > 0
         if n == 1:
@@ -104,17 +102,15 @@ def test_launch_params_report_the_launched_geometry(tmp_path):
         elif n <= 32:
             assert (g, b, r, t) == (32, 1024, 4, 128)
             assert s > 0
-        elif n <= 128:
-            nb = math.ceil(n / 32)
-            assert (g, r, t) == (32 * nb * nb, 1, 32 * nb * nb), n
-            assert 0 < b <= 4096
         else:
-            split = 2 if n <= 240 else (4 if n <= 256 else (2 if n <= 512 else 1))
-            th = min(1024, math.ceil(n / 32) * 32 * split)
-            assert (g, r, t) == (th, 1, th), n
-            assert 0 < b <= 4096
+            warps, blocks = next(x[1:] for x in ((64, 1, 1), (96, 2, 1), (160, 4, 1), (256, 8, 1), (352, 8, 2),
+                                                 (512, 8, 4), (736, 8, 8), (1024, 8, 16)) if n <= x[0])
+            assert (g, r, t) == (32 * warps * blocks, 1, 32 * warps), n
+            assert 0 < b <= 4096 * blocks and b % blocks == 0 and s > 0
+    import torch
     import eigeng_b200 as E
     assert E.launch_params(4096, 128)["numTH"] == rows[128][3]
+    assert E.launch_params(4096, 64, torch.float32)["grpSZ"] == 128
     E.tune_set([dict(esize=8, n=256, split=0, zmem=0, ql_mpw=0, reduce=E.REDUCE_CLUSTER)])
     try:
         lp = E.launch_params(4096, 256)
