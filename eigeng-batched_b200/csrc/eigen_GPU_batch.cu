@@ -628,9 +628,10 @@ cudaError_t run(long L, int nm, int n, int m, T *a, T *w, void *wk, size_t lwork
   const int k1c_nt = k1c_threads<T>(n);
   const int red_form = tuned_reduce((int)sizeof(T), n);
   const bool k1_cluster = red_form == EIGEN_GPU_REDUCE_CLUSTER && k1cl_usable<T>(n, dp);
-  const bool k1_in_regs = !k1_cluster && reg_form<T>(n);
+  const bool k1_staged = red_form == EIGEN_GPU_REDUCE_STAGED;
+  const bool k1_in_regs = !k1_cluster && !k1_staged && reg_form<T>(n);
   const SymCfg k1_symc = sym_cfg<T>(n);
-  const bool k1_symm = !k1_cluster && sym_usable<T>(n, k1_symc, dp);
+  const bool k1_symm = !k1_cluster && !k1_staged && sym_usable<T>(n, k1_symc, dp);
   const FormQ<T> k1_fq = form_q_cfg<T>(n, (size_t)dp.smem_optin);
   const size_t k1c_smem = k1_in_regs ? k1r_smem_bytes<T>(n) : sizeof(T) * k1c_smem_elems(n, k1c_nt, pl.k1b);
   size_t k3c_smem = k3c_smem_bytes<T>(n, ztm ? 0 : pl.zrows);
@@ -865,12 +866,13 @@ cudaError_t launch_params(long L, int n, int *grp, int *tb, int *gr, int *th, in
     *th = 32 * K1W_NW;
     *tb = (int)((lc + K1W_NW - 1) / K1W_NW);
     *sh = (int)(sizeof(T) * tw_smem_elems() * K1W_NW);
-  } else if (reg_form<T>(n)) {  // k1_reg: 2 x 2 warps
+  } else if (reg_form<T>(n) && red_form != EIGEN_GPU_REDUCE_STAGED) {  // k1_reg: 2 x 2 warps
     *grp = *th = 32 * 4;
     *gr = 1;
     *tb = (int)lc;
     *sh = (int)k1r_smem_bytes<T>(n);
-  } else if (const SymCfg c = sym_cfg<T>(n); sym_usable<T>(n, c, dp)) {  // k1_sym, its launch on the whole matrices
+  } else if (const SymCfg c = sym_cfg<T>(n); red_form != EIGEN_GPU_REDUCE_STAGED && sym_usable<T>(n, c, dp)) {
+    // k1_sym, its launch on the whole matrices
     *th = 32 * c.nw;
     *grp = c.cn * *th;
     *gr = 1;
@@ -2730,7 +2732,7 @@ cudaError_t eigen_GPU_batch_tune_set(const eigen_GPU_tune_entry *entries, const 
     const eigen_GPU_tune_entry &e = entries[i];
     if ((e.esize != 4 && e.esize != 8) || e.n < 1 || e.n > 1024 || e.split < 0 || e.split > 32 ||
         (e.zmem != EIGEN_GPU_ZMEM_AUTO && e.zmem != EIGEN_GPU_ZMEM_SHARED) || e.ql_mpw < 0 || e.ql_mpw > 32 ||
-        (e.ql_mpw & (e.ql_mpw - 1)) != 0 || e.reduce < EIGEN_GPU_REDUCE_AUTO || e.reduce > EIGEN_GPU_REDUCE_CLUSTER)
+        (e.ql_mpw & (e.ql_mpw - 1)) != 0 || e.reduce < EIGEN_GPU_REDUCE_AUTO || e.reduce > EIGEN_GPU_REDUCE_STAGED)
       return cudaErrorInvalidValue;
   }
   std::lock_guard<std::mutex> lk(eigb::g_mu);

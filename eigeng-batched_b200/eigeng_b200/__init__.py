@@ -22,7 +22,7 @@ LIB_PATH = os.path.join(os.path.dirname(_HERE), "lib", "libeigenGbatch.so")
 
 TQL2, IMTQL2, JACOBI = 0, 1, 2
 ZMEM_AUTO, ZMEM_SHARED = 0, 1  # where the apply phase keeps Z (eigen_GPU_batch_opts.zmem)
-REDUCE_AUTO, REDUCE_CTA, REDUCE_CLUSTER = 0, 1, 2  # phase-1 kernel (eigen_GPU_tune_entry.reduce)
+REDUCE_AUTO, REDUCE_CTA, REDUCE_CLUSTER, REDUCE_STAGED = 0, 1, 2, 3  # phase-1 kernel (eigen_GPU_tune_entry.reduce)
 # phases of eigen_GPU_batch_stage_* (EIGEN_GPU_STAGE_*)
 STAGE_REDUCE, STAGE_QL, STAGE_APPLY, STAGE_ALL = 1, 2, 4, 7
 

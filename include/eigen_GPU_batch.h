@@ -390,18 +390,22 @@ typedef struct eigen_GPU_tune_entry {
   int split;  /* 0: automatic, else as eigen_GPU_batch_opts.split (1..32) */
   int zmem;   /* EIGEN_GPU_ZMEM_AUTO or EIGEN_GPU_ZMEM_SHARED */
   int ql_mpw; /* 0: automatic, else a power of two 1..32 */
-  int reduce; /* phase-1 kernel: EIGEN_GPU_REDUCE_AUTO, _CTA or _CLUSTER */
+  int reduce; /* phase-1 kernel: EIGEN_GPU_REDUCE_AUTO, _CTA, _CLUSTER or _STAGED */
 } eigen_GPU_tune_entry;
 /* phase-1 kernels: automatic, which is also what _CTA asks for (one warp or
  * CTA per matrix while its upper triangle fits one multiprocessor, the
- * fewest CTAs that hold it above: FP64 n > 256, FP32 n > 384), or a
+ * fewest CTAs that hold it above: FP64 n > 256, FP32 n > 384); a
  * thread-block cluster holding the whole matrix in distributed shared memory
- * (32 < n <= 512, where the device can run it; measured slower on B200).
+ * (32 < n <= 512, where the device can run it; measured slower on B200); or,
+ * for n > 32, one CTA per matrix with a leading block staged in shared memory
+ * and the rest in global memory, which automatic falls back to on a device
+ * that cannot run its cluster (B200, FP64 n=256 L=2048: 51 ms, automatic 11).
  * Unlike the other entries, the choice changes rounding (another summation
  * order), within the solver's accuracy. */
 #define EIGEN_GPU_REDUCE_AUTO 0
 #define EIGEN_GPU_REDUCE_CTA 1
 #define EIGEN_GPU_REDUCE_CLUSTER 2
+#define EIGEN_GPU_REDUCE_STAGED 3
 cudaError_t eigen_GPU_batch_tune_set(const eigen_GPU_tune_entry *entries, const int count);
 cudaError_t eigen_GPU_batch_tune_get(const int esize, const int n, eigen_GPU_tune_entry *out);
 
