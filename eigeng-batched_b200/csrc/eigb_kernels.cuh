@@ -35,7 +35,6 @@
 #pragma once
 #include <stdio.h>
 
-#include "eigb_apply.cuh"  // host-tested only
 #include "eigb_common.cuh"
 #include "eigb_formq.cuh"
 #include "eigb_ql.cuh"

@@ -25,6 +25,7 @@ namespace simt {
 struct Barrier {
   int need = 0, here = 0;
   long gen = 0;
+  bool any = false, last_any = false;  // of the arrivals, and of the last round
 };
 struct Fiber {
   ucontext_t ctx;  // its first entry; later switches by jumps, which make no system call
@@ -64,6 +65,8 @@ inline void block(Barrier &b)  // arrives; returns when all have
 {
   if (++b.here == b.need) {
     b.here = 0;
+    b.last_any = b.any;
+    b.any = false;
     b.gen++;
     return;
   }
@@ -169,6 +172,8 @@ struct NDim {
 
 }  // namespace simt
 
+#undef __shared__
+#define __shared__ static  // one CTA at a time
 #define threadIdx (simt::Dim())
 #define blockIdx (simt::BDim())
 #define blockDim (simt::NDim())
@@ -182,6 +187,14 @@ inline int __any_sync(unsigned, int p)
 }
 inline void __syncwarp() { simt::block(simt::cta().warps[simt::m->cur->tid >> 5].bar); }
 inline void __syncthreads() { simt::block(simt::cta().bar); }
+inline int __syncthreads_or(int p)
+{
+  simt::Barrier &b = simt::cta().bar;
+  b.any = b.any || p;
+  simt::block(b);
+  return b.last_any;
+}
+inline int __clz(int x) { return x ? __builtin_clz((unsigned)x) : 32; }
 template <class T> T min(T a, T b) { return b < a ? b : a; }
 template <class T> T max(T a, T b) { return a < b ? b : a; }
 

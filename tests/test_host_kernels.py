@@ -1,8 +1,10 @@
 """CPU unit tests of the library's own device code compiled for the host:
-the phase-2 QL rotation generator (eigb_ql.cuh) and the phase-1 team code
+the phase-2 QL rotation generator (eigb_ql.cuh), the phase-1 team code
 (eigb_tridiag.cuh, run by one std::thread per GPU thread with std::barrier
-for the CTA barrier).  They check the algorithms against the oracle without
-a GPU; the -m gpu tests check the compiled kernels."""
+for the CTA barrier) and phase 3 (the pairs of sweeps of eigb_kernels.cuh; the
+wave of eigb_wave.cuh on fibers, tests/host/simt.hpp).  They check the
+algorithms against the oracle without a GPU; the -m gpu tests check the compiled
+kernels."""
 import ctypes
 import os
 import subprocess
@@ -38,9 +40,22 @@ def hostlibs():
         f.restype = I
         getattr(libs["tridiag_host"], "host_tridiag" + s).argtypes = [I, I, I, P, I, I, P, P]
         getattr(libs["tridiag_host"], "host_tridiag_reg" + s).argtypes = [I, P, I, P, P]
-        getattr(libs["apply_host"], "host_apply" + s).argtypes = [I, P, P, I, I, I]
+        getattr(libs["apply_host"], "host_apply" + s).argtypes = [I, P, P, I, I]
         getattr(libs["apply_host"], "host_apply" + s).restype = I
     return libs
+
+
+@pytest.fixture(scope="module")
+def wavelib():
+    out = os.path.join(tempfile.mkdtemp(prefix="eigb_wave_"), "libwave_host.so")
+    subprocess.check_call(["g++", "-x", "c++", "-std=c++20", "-O1", "-ffp-contract=off", "-Wno-unknown-pragmas", "-fPIC",
+                           "-U_FORTIFY_SOURCE",  # it takes jumps between stacks for an error
+                           "-shared", "-I/usr/local/cuda/include", "-o", out, os.path.join(HOST, "wave_host.cu")])
+    so = ctypes.CDLL(out)
+    P, I = ctypes.c_void_p, ctypes.c_int
+    for f in (so.host_wave_d, so.host_wave_f):
+        f.restype, f.argtypes = ctypes.c_long, [I, P, I, I, I, I, P, I, P, I, P]
+    return so
 
 
 def _p(x):
@@ -223,10 +238,11 @@ def test_fast_generator_is_bit_identical(oracle_mod, hostlibs, n, method, dtype)
 @pytest.mark.parametrize("n", [3, 8, 17, 33, 64, 100])
 @pytest.mark.parametrize("method", [0, 1])
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
-def test_pipelined_apply_matches_sequential(oracle_mod, hostlibs, n, method, dtype):
+def test_pipelined_apply_matches_sequential(oracle_mod, hostlibs, wavelib, n, method, dtype):
     """Phase 3 applies each sweep as one rotation chain whose operands are
     loaded a block ahead; the result equals applying every rotation in
-    order, also when the stream is staged in small chunks."""
+    order, also when the stream is staged in small chunks.  The wave form,
+    16 sweeps at a time, gives the same bits."""
     O = oracle_mod
     a0 = O.sym_uniform(1, n, seed=7 * n + method)[0].astype(dtype)
     d, e = tred(O, a0, n)
@@ -240,15 +256,20 @@ def test_pipelined_apply_matches_sequential(oracle_mod, hostlibs, n, method, dty
     flat = np.ascontiguousarray(rec)
     eps = np.finfo(dtype).eps
     first = None
-    for kg in (0, 2, 4, 8):
-        for ch in (4 * (n + 1), n + 1, 10 ** 6):
-            z = np.ascontiguousarray(q0.copy())
-            segs = f(n, _p(z), _p(flat), flat.shape[0], ch, kg)
-            assert segs > 0
-            assert np.abs(z - ref).max() <= 64 * n * eps * np.abs(ref).max()
-            # chunking and the group size change which sweeps are applied
-            # together; the pipelines do the same operations in the same
-            # order, so the results are identical
-            if first is None:
-                first = z
-            assert np.array_equal(z, first), (kg, ch)
+    for ch in (4 * (n + 1), n + 1, 10 ** 6):
+        z = np.ascontiguousarray(q0.copy())
+        segs = f(n, _p(z), _p(flat), flat.shape[0], ch)
+        assert segs > 0
+        assert np.abs(z - ref).max() <= 64 * n * eps * np.abs(ref).max()
+        # chunking changes which sweeps are applied together; the pairs do
+        # the same operations in the same order, so the results are identical
+        if first is None:
+            first = z
+        assert np.array_equal(z, first), ch
+    # the wave form of phase 3: 16 sweeps at a time, each row the same
+    # operations in the same order, for one and two rows a thread
+    fw = getattr(wavelib, "host_wave_d" if dtype == np.float64 else "host_wave_f")
+    for rows in (1, 2):
+        a = np.asfortranarray(q0)
+        assert fw(rows, _p(a), n, n, 0, n, _p(flat), flat.shape[0], _p(dq), 0, None) == 0
+        assert np.array_equal(a, first), rows
