@@ -872,7 +872,7 @@ def main():
     # record counts (mean rotations per matrix) for the algorithmic byte model
     recs = 1.1 * n * n
     pb = phase_bytes(n, esize, recs)
-    names = ["tridiag_qt", "ql_rotations", "apply_rotations"]
+    names = ["reduction_q", "ql_rotations", "apply_rotations"]
     dom = int(np.argmax(ph))
     achieved = pb[dom] * L / (ph[dom] / 1000.0) / 1e9 if ph[dom] > 0 else 0.0
     traffic = measured_traffic(names[dom], args.dtype, n)

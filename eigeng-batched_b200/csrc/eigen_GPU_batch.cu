@@ -174,10 +174,12 @@ template <class T> size_t k2_smem_per_thread(int n) { return sizeof(T) * 2 * (si
 // power of two that is.  Each warp alone is bound by its chains' latency, up
 // to about one warp a scheduler; beyond, more lanes a warp cost less than
 // more warps.  Measured on B200 (phase 2, ms by matrices per warp): FP64 n=256
-// L=2048 1: 13.5, 2: 9.1, 4: 7.3, 8: 8.0; n=128 L=4096 4: 2.25, 8: 1.77, 16:
-// 1.91; n=45 L=6000 8: 0.46, 16: 0.37; n=512 L=256 1: 21.1, 2: 24.3; FP32
-// n=201 L=1000 1: 2.85, 2: 3.49; n=256 L=2048 2: 5.5, 4: 5.2, 8: 5.9.  (Taken
-// before the rotation loop was unrolled, which scales them alike.)
+// L=2048 1: 9.8, 2: 6.0, 4: 5.0, 8: 5.4; n=256 L=592 1: 3.9, 2: 4.4; L=593 1:
+// 5.2, 2: 4.4, 4: 4.9; n=128 L=4096 4: 1.91, 8: 1.56, 16: 1.68; n=45 L=6000 8:
+// 0.36, 16: 0.30; n=512 L=256 1: 14.2, 2: 16.3; FP32 n=256 L=1184 1: 2.83, 2:
+// 2.67, 4: 3.07; L=1185 1: 3.81, 2: 3.35, 4: 3.07; L=2048 2: 3.44, 4: 3.08, 8:
+// 3.48; n=201 L=1000 1: 1.83, 2: 1.73.  (In FP32 two would be 6 % better than
+// one from L = 1000 to 1184.)
 template <class T> int k2_mpw(long L, int sms)
 {
   if (L <= (sizeof(T) == 8 ? 4L : 8L) * sms) return 1;

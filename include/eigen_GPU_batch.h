@@ -79,8 +79,9 @@ typedef struct eigen_GPU_batch_opts {
   int zmem;      /* EIGEN_GPU_ZMEM_AUTO (0; any other value but
                     EIGEN_GPU_ZMEM_SHARED means the same) or EIGEN_GPU_ZMEM_SHARED */
   int ql_mpw;    /* QL phase: matrices per warp (one per lane), a power of
-                    two 1..32; <= 0: automatic (about three warps per SM;
-                    fewer per warp spread a small batch over more warps).
+                    two 1..32; <= 0: automatic (one while that is at most
+                    four warps per SM, eight in FP32, else as many as
+                    keep to four).
                     Solves that run concurrently on other streams do
                     better with 4..8: fewer warps then take issue slots
                     from the other solve's kernels.  Results do not
@@ -308,8 +309,8 @@ cudaError_t eigen_GPU_batch_interleaved_FP(const int L, const int n, const float
  * also caps the matrices of a wave, and so the workspace).  In each wave
  * the groups' reductions run concurrently on internal streams, then one
  * persistent launch runs the QL phase of every matrix of the wave from a
- * device work queue (longest first, opts->ql_mpw matrices per warp, 4 by
- * default), then the groups' apply phases run concurrently again.  The call
+ * device work queue (longest first, opts->ql_mpw matrices per warp; automatic:
+ * up to 4), then the groups' apply phases run concurrently again.  The call
  * is asynchronous with respect to the host except for small index copies
  * from host memory, and the caller's stream waits for all of it.  Results
  * equal eigen_GPU_batch_ex_* on each matrix, bit for bit.  Other options as
