@@ -955,8 +955,8 @@ __global__ void __launch_bounds__(SM ? 256 : 512, 1) k3_cta(const KP<T> p)
 // Phase 3, wave form: p.wrows rows of one matrix per CTA, 32 R rows per
 // warp and one more warp that stages the records.  Bound by the latency of the
 // rotation chains between their record loads and by FP64 issue (n=256 FP64:
-// FP64 pipe 52 % active, waits for record loads and for fixed latency 2.6
-// cycles an instruction), so by warps in flight: MB bounds the registers, U
+// FP64 pipe 52 % active; waits for fixed latency, column loads and barriers 1.4,
+// 1.4 and 1.1 cycles an instruction), so by warps in flight: MB bounds the registers, U
 // the columns in flight that those pay for.  B200, phase 3, ms: FP64 n=256
 // L=2048 two rows per thread, two CTAs an SM and U = 4 14.5, three and U = 2
 // 14.0, one row, four CTAs 16.1; n=144 L=3000 6.93, 6.18, 7.67.
