@@ -59,9 +59,11 @@ template <class T> SymCfg sym_cfg(int n)
 //    without / at the order given:) FP64 n=400 256: L=500 21.4 / 15.6, L=4 1.27 /
 //    1.42; n=512 256: L=256 17.6 / 14.6, L=4 1.98 / 2.14; n=736 512, 256: L=64
 //    19.4 / 14.3, L=4 3.53 / 3.78; n=1000 736, 512, 256: L=32 30.1 / 21.5, L=4
-//    5.97 / 6.42.  Also 352: n=512 L=256 14.0, but L=4 2.38.  FP32 n=400 160:
-//    L=500 12.6 / 11.1, L=4 1.26 / 1.26 (384, 160: 10.3, 1.54); n=736 160: L=100
-//    18.5 / 17.8, L=4 3.22 / 3.23; n=1000 736: L=32 19.7 / 14.8, L=4 5.78 / 5.98.
+//    5.97 / 6.42.  Also 352: n=512 L=256 14.0, but L=4 2.38.  FP32 n=400 384:
+//    L=500 12.6 / 10.7, L=4 1.26 / 1.49; n=512 384: L=256 11.5 / 10.1, L=4 2.00 /
+//    2.22; n=736 384: L=100 18.5 / 16.5, L=4 3.22 / 3.57; n=1000 736: L=32 19.7 /
+//    14.8, L=4 5.78 / 5.98.  At 256 or 160 instead the solve of n=400 L=400 takes
+//    4 or 5 % longer than with 384 (19.3 ms), that of L=4 1 or 3 % less.
 template <class T> int sym_next(int n, long cnt, int sms)
 {
   const SymCfg c = sym_cfg<T>(n);
@@ -70,7 +72,7 @@ template <class T> int sym_next(int n, long cnt, int sms)
     if (c.cn > 1) return n > 736 ? 736 : (n > 512 ? 512 : 256);
     return wave ? (n > 128 ? 128 : (n > 64 ? 64 : 0)) : 0;
   }
-  if (c.cn > 1) return n > 736 ? 736 : 160;
+  if (c.cn > 1) return n > 736 ? 736 : 384;
   return wave && n > 160 ? 160 : 0;
 }
 
